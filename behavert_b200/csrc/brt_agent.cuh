@@ -710,6 +710,15 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
   return n;
 }
 
+// The agent (sorted slot) of this lane when a warp takes `warpAgents`
+// consecutive agents, one in each of its first lanes; false for the lanes
+// without one.
+__device__ __forceinline__ bool agentOfLane(uint32_t warpAgents, uint32_t n, uint32_t& slot) {
+  const uint32_t lane = threadIdx.x & 31u, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  slot = warp * warpAgents + lane;
+  return lane < warpAgents && slot < n;
+}
+
 // Home-agent context for the steering stages.
 struct AgentCtx {
   f3 pos, fwd;

@@ -236,6 +236,7 @@ StageArgs stageArgs(brt_engine* e) {
   A.flocks = e->flocks; A.agentBase = e->agentBase; A.obstacles = e->obstacles; A.obsMask = e->obsMask;
   A.lists = e->lists; A.listStride = e->listStride;
   A.nflocks = e->nflocks; A.n = e->N; A.Fs = e->Fs;
+  A.warpAgents = e->listsWarp;
   A.stepCounter = e->stepCounter;
   return A;
 }
@@ -373,6 +374,9 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   bool twoPass = e->forceTwoPass || (e->anyKnn && e->Mmax > 32);
   for (const FlockDev& d : e->flocksHost) twoPass = twoPass || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
   if (e->anyKnn && !twoPass) F.scanVariant = 8;
+  F.warpAgents = e->school ? e->schoolWarp
+                 : twoPass ? e->fusedWarp
+                           : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);
   if (e->school) BRT_CUDA_TRY(launchSchool(F, e->stream));
   else if (twoPass) BRT_CUDA_TRY(launchFused(F, e->anyKnn, e->stream));
   else BRT_CUDA_TRY(launchFlock(F, e->phase2Variant, e->fusedBlock, e->regBudget, e->stream));
@@ -1593,6 +1597,9 @@ int configureKernels(brt_engine* e) {
   BRT_CUDA_TRY(configureFusedKernels(mx));
   BRT_CUDA_TRY(configureFlockKernels(mx));
   BRT_CUDA_TRY(configureSchoolKernels(mx));
+  e->listsWarp = listsWarpAgents(e->N, e->Mmax, e->smCount);
+  e->fusedWarp = fusedWarpAgents(e->N, e->Mmax, e->smCount);
+  e->schoolWarp = schoolWarpAgents(e->N, e->Mmax, e->smCount);
   return BRT_OK;
 }
 }  // namespace

@@ -39,6 +39,8 @@ struct brt_engine {
   // 1M-agent flock and the 1,024-flock batch.
   int phase2Variant = 2;      // option "phase2_variant": list walk shape (2: geometry, then features)
   int scanVariant = 5;        // option "scan_variant": neighbour-scan loop shape (5: warp-cooperative, windowed)
+  // agents a warp of listsKernel, fusedKernel and schoolKernel takes (warpAgentsFor)
+  uint32_t listsWarp = 32, fusedWarp = 32, schoolWarp = 32;
   // scan variant 6: the (flock, row segment) tiles of the staged tile kernel
   uint4* tiles = nullptr;
   uint32_t numTiles = 0;

@@ -225,11 +225,11 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
 template <int FP, int P2, int MINB, int SCAN>
 __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs A) {
   extern __shared__ __align__(16) uint32_t sList[];
-  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i0 < A.n;
   // The warp-cooperative scans need every lane of the warp; inactive lanes
   // take part read-only (mirroring the last agent) and leave after it.
   constexpr bool coop = SCAN != 0;
+  uint32_t i0;
+  const bool active = coop ? agentOfLane(A.warpAgents, A.n, i0) : (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n;
   if (!coop && !active) return;
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
@@ -593,6 +593,15 @@ uint32_t tileFlockBlocks(uint32_t Mmax, uint32_t Fs, int smCount) {
   return (uint32_t)(per * std::max(1, smCount));
 }
 
+// Resident warps: what the register budget allows (flockKernel's launch
+// bounds), or the lists' shared memory.
+uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount) {
+  const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+  const size_t smem = flockSmemBytes(block, A.Mmax, A.scanVariant) + 1024;
+  const uint32_t bySmem = (uint32_t)(228u * 1024u / smem) * (block / 32u);
+  return warpAgentsFor(A.n, smCount * std::min(byRegs, bySmem));
+}
+
 cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   if (A.scanVariant == 6) {
@@ -605,7 +614,8 @@ cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs
     return launchTileFP<32>(A, phase2, st);
   }
   if (block < 32 || block > kFlockMaxThreads || block % 32) return cudaErrorInvalidValue;
-  const uint32_t blocks = (A.n + block - 1) / block;
+  const uint32_t blockAgents = A.scanVariant >= 4 ? block / 32 * A.warpAgents : block;
+  const uint32_t blocks = (A.n + blockAgents - 1) / blockAgents;
   const uint32_t fp = A.Fs;
   const size_t smem = flockSmemBytes(block, A.Mmax, A.scanVariant);
   if (fp == 0) return launchFlockFP<0>(A, blocks, block, smem, phase2, regs, st);

@@ -156,8 +156,8 @@ __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, ui
 template <bool KNN>
 __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
-  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i0 < A.n;
+  uint32_t i0;
+  const bool active = KNN ? (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n : agentOfLane(A.warpAgents, A.n, i0);
   if (KNN && !active) return;
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
@@ -225,8 +225,8 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
 template <bool KNN>
 __global__ void __launch_bounds__(128) listsKernel(StageArgs A) {
   extern __shared__ uint32_t sList[];
-  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i0 < A.n;
+  uint32_t i0;
+  const bool active = KNN ? (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n : agentOfLane(A.warpAgents, A.n, i0);
   if (KNN && !active) return;
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
@@ -385,17 +385,33 @@ cudaError_t configureFusedKernels(uint32_t Mmax) {
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(listsKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(129 * Mmax * 4));
 }
+namespace {
+uint32_t residentWarpAgents(const void* fn, int threads, size_t smem, uint32_t n, uint32_t smCount) {
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem) != cudaSuccess || per < 1) {
+    cudaGetLastError();
+    per = 1;
+  }
+  return warpAgentsFor(n, smCount * (uint32_t)(per * threads / 32));
+}
+}  // namespace
+uint32_t fusedWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
+  return residentWarpAgents((const void*)fusedKernel<false>, kFusedThreads, (size_t)(kFusedThreads + 1) * Mmax * 4, n, smCount);
+}
+uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
+  return residentWarpAgents((const void*)listsKernel<false>, 128, (size_t)129 * Mmax * 4, n, smCount);
+}
 cudaError_t launchFused(const FusedArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const size_t smem = (size_t)(kFusedThreads + 1) * A.Mmax * 4;
   if (knn) fusedKernel<true><<<blocksFor(A.n, kFusedThreads), kFusedThreads, smem, st>>>(A);
-  else fusedKernel<false><<<blocksFor(A.n, kFusedThreads), kFusedThreads, smem, st>>>(A);
+  else fusedKernel<false><<<blocksFor(A.n, kFusedThreads / 32 * A.warpAgents), kFusedThreads, smem, st>>>(A);
   return cudaGetLastError();
 }
 cudaError_t launchLists(const StageArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   if (knn) listsKernel<true><<<blocksFor(A.n, 128), 128, 0, st>>>(A);
-  else listsKernel<false><<<blocksFor(A.n, 128), 128, (size_t)129 * (A.listStride - 1) * 4, st>>>(A);
+  else listsKernel<false><<<blocksFor(A.n, 128 / 32 * A.warpAgents), 128, (size_t)129 * (A.listStride - 1) * 4, st>>>(A);
   return cudaGetLastError();
 }
 // Registered per-agent arrays of `words` 32-bit words: slot i of dst takes

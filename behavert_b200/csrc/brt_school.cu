@@ -153,8 +153,8 @@ __device__ __forceinline__ void copyFeatures(const float* featS, float* featA, u
 // the last agent read-only and leave after the scan.
 __global__ void __launch_bounds__(128) schoolKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
-  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i0 < A.n;
+  uint32_t i0;
+  const bool active = agentOfLane(A.warpAgents, A.n, i0);
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
   const FlockDev& fl = A.flocks[f];
@@ -226,9 +226,18 @@ __global__ void __launch_bounds__(128) schoolStageKernel(StageArgs A, int which)
 
 cudaError_t launchSchool(const FusedArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
-  const uint32_t block = 128;
-  schoolKernel<<<(A.n + block - 1) / block, block, (size_t)(block + 1) * A.Mmax * 4, st>>>(A);
+  const uint32_t block = 128, blockAgents = block / 32 * A.warpAgents;
+  schoolKernel<<<(A.n + blockAgents - 1) / blockAgents, block, (size_t)(block + 1) * A.Mmax * 4, st>>>(A);
   return cudaGetLastError();
+}
+
+uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, schoolKernel, 128, (size_t)129 * Mmax * 4) != cudaSuccess || per < 1) {
+    cudaGetLastError();
+    per = 1;
+  }
+  return warpAgentsFor(n, smCount * (uint32_t)(per * 4));
 }
 
 cudaError_t launchSchoolStage(const StageArgs& A, int which, cudaStream_t st) {
