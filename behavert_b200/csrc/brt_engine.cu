@@ -176,12 +176,10 @@ cudaError_t launchIota(uint32_t* a, uint32_t n, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The re-sort's state as after creation: no previous order, empty mover
-// lists (kNoMover heads), zero counters and look-back words.
-cudaError_t resetResort(brt_engine* e) {
-  cudaError_t err = cudaMemsetAsync(e->resortMem, 0, e->resortWords * 4, e->stream);
-  if (err == cudaSuccess && e->C) err = cudaMemsetAsync(e->rsHead, 0xFF, (size_t)e->C * 4, e->stream);
-  return err;
+// The cell counts as between steps (the cell scan leaves them at zero; a step
+// whose waits ran out may have placed agents by other starts, nothing else).
+cudaError_t resetOrder(brt_engine* e) {
+  return cudaMemsetAsync(e->orderCount, 0, (size_t)e->Cpad * 4, e->stream);
 }
 
 void freeAll(brt_engine* e) {
@@ -195,7 +193,7 @@ void freeAll(brt_engine* e) {
   void* ptrs[] = {e->flocks, e->agentBase, e->obstacles, e->obsMask, e->posA, e->fwdA, e->accA, e->posS, e->fwdS, e->accS,
                   e->featA, e->featS, e->idA, e->idS, e->statsById, e->steer, e->lists, e->pairs[0], e->pairs[1],
                   e->cellStart, e->cellEnd, e->sortMem, e->errWord, e->stage4, e->stageF, e->stepCounter, e->cullWords,
-                  e->membership[0], e->membership[1], e->resortMem};
+                  e->membership[0], e->membership[1], e->cellPlace, e->members, e->orderCount, e->orderMem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->tiles) cudaFree(e->tiles);
@@ -262,53 +260,39 @@ int stageMark(brt_engine* e, int k) {
   return BRT_OK;
 }
 
-// hash -> sort -> reorder + cell ranges
-ResortArgs resortArgs(brt_engine* e) {
-  ResortArgs A{};
-  A.pos = e->posA; A.id = e->idA; A.prevPairs = e->pairs[e->plan.passes & 1];
-  A.cellStart = e->cellStart; A.cellEnd = e->cellEnd;
+OrderArgs orderArgs(brt_engine* e) {
+  OrderArgs A{};
+  A.pos = e->posA; A.id = e->idA;
   A.flocks = e->flocks; A.agentBase = e->agentBase;
   A.nflocks = e->nflocks; A.n = e->N; A.numCells = e->C;
-  A.maxMovers = e->N / 8;
-  A.newKey = e->rsNewKey; A.prefix = e->rsPrefix; A.blockStay = e->rsBlockStay;
-  A.moverCount = e->rsCount; A.moverHead = e->rsHead; A.moverNext = e->rsNext;
-  A.newStart = e->rsNewStart; A.stayBase = e->rsStayBase; A.tileStatus = e->rsTiles; A.tileCounter = e->rsCounter; A.words = e->rsWords;
+  A.cellPlace = e->cellPlace; A.count = e->orderCount;
+  A.cellStart = e->cellStart; A.cellEnd = e->cellEnd;
+  A.members = e->members;
+  A.scratch[0] = e->pairs[0]; A.scratch[1] = e->pairs[1];
+  A.words = e->orderMem; A.bigCells = e->orderMem + kOrderWords;
+  A.tileStatus = A.bigCells + bigCellCap(e->N);
   A.stepCounter = e->stepCounter;
-  A.out = e->pairs[e->plan.passes & 1];
   A.errWord = e->errWord;
   A.wait = e->wait;
   return A;
 }
 
-// The next fused step cannot take its order from the current one (the
-// canonical arrays or the sort plan were replaced): it runs the full sort.
-cudaError_t invalidateResort(brt_engine* e) {
-  return cudaMemsetAsync(e->rsWords + kResortWordValid, 0, 4, e->stream);
-}
-
-// Hash, sort and reorder.  From the fused step (incremental) the order comes
-// from the incremental re-sort when the previous step's order allows it, the
-// hash and radix passes running only otherwise (decided on the device).
-int enqueueReorder(brt_engine* e, bool incremental = false) {
+// Order and reorder: by counting the cells, or with the radix sort.
+int enqueueReorder(brt_engine* e) {
   cudaStream_t st = e->stream;
   int rc = stageMark(e, 0);
   if (rc) return rc;
-  const bool rs = incremental && e->resortOn;
-  HashArgs H = hashArgs(e);
-  H.resortValid = e->rsWords + kResortWordValid;
-  const uint32_t* gate = nullptr;
-  ResortArgs RS;
-  if (rs) {
-    RS = resortArgs(e);
-    BRT_CUDA_TRY(launchResortMark(RS, st));
-    gate = e->rsWords + kResortWordMode;
-    H.gate = gate;
+  if (e->orderByCount) {
+    const OrderArgs O = orderArgs(e);
+    BRT_CUDA_TRY(launchOrderCount(O, st));
+    if ((rc = stageMark(e, 1))) return rc;
+    BRT_CUDA_TRY(launchOrderPlace(O, st));
+  } else {
+    BRT_CUDA_TRY(launchHash(hashArgs(e), e->smCount * 8, st));
+    if ((rc = stageMark(e, 1))) return rc;
+    for (uint32_t k = 0; k < e->plan.passes; ++k)
+      BRT_CUDA_TRY(launchOnesweepPass(e->plan, k, e->pairs[k & 1], e->pairs[(k + 1) & 1], e->ss, e->errWord, st));
   }
-  BRT_CUDA_TRY(launchHash(H, e->smCount * 8, st));
-  if ((rc = stageMark(e, 1))) return rc;
-  for (uint32_t k = 0; k < e->plan.passes; ++k)
-    BRT_CUDA_TRY(launchOnesweepPass(e->plan, k, e->pairs[k & 1], e->pairs[(k + 1) & 1], e->ss, e->errWord, st, gate));
-  if (rs) BRT_CUDA_TRY(launchResortPlace(RS, st));
   if ((rc = stageMark(e, 2))) return rc;
   e->finalPairs = e->plan.passes & 1;
   ReorderArgs R;
@@ -325,11 +309,9 @@ int enqueueReorder(brt_engine* e, bool incremental = false) {
     R.cullWords = e->cullWords;
     R.flocks = e->flocks; R.agentBase = e->agentBase; R.nflocks = e->nflocks;
   }
-  if (rs) {
-    R.resortMode = e->rsWords + kResortWordMode;
-    R.newStart = e->rsNewStart;
-    R.moverCount = e->rsCount; R.moverHead = e->rsHead;
-    R.resortValid = e->rsWords + kResortWordValid;
+  if (e->orderByCount) {
+    R.members = e->members;
+    R.pairsOut = e->pairs[e->finalPairs];
   }
   BRT_CUDA_TRY(launchReorder(R, st));
   // registered arrays move with their agents (slot i takes the previous slot
@@ -353,7 +335,7 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
     int rc = drainSlot(e, e->ringPos);
     if (rc) return rc;
   }
-  int rc = enqueueReorder(e, true);
+  int rc = enqueueReorder(e);
   if (rc) return rc;
   FusedArgs F;
   std::memset(&F, 0, sizeof(F));
@@ -459,7 +441,6 @@ int buildTiles(brt_engine* e) {
 
 namespace brt {
 int engineEnqueueStep(brt_engine* e, float dt, bool record) { return enqueueStep(e, dt, record); }
-cudaError_t engineInvalidateResort(brt_engine* e) { return invalidateResort(e); }
 int engineSyncAndCheck(brt_engine* e) { return syncAndCheck(e); }
 }  // namespace brt
 
@@ -609,21 +590,10 @@ int brt_engine_create(const brt_params* flocks, uint32_t num_flocks, int device,
   chk(devAlloc(&e->stageF, std::max<size_t>(1, n * e->Fmax)));
   const size_t sortBytes = sortScratchBytes(e->plan, false);
   if (!rc && cudaMalloc(&e->sortMem, sortBytes) != cudaSuccess) { setLastError("sort scratch allocation failed"); rc = BRT_ERR_CUDA; }
-  // incremental re-sort arrays, each on a 16-byte boundary
-  auto words4 = [](size_t w) { return (w + 3) & ~(size_t)3; };
-  const size_t rsSizes[11] = {n, n, n, (size_t)resortBlocks(e->N) + 1, e->C, e->C, e->C,
-                              std::max<size_t>(1, resortCellTiles(e->C)), 1, kResortWords, e->C};
-  size_t rsWordsTotal = 0;
-  for (size_t w : rsSizes) rsWordsTotal += words4(w);
-  if (!rc && cudaMalloc(&e->resortMem, rsWordsTotal * 4) != cudaSuccess) { setLastError("re-sort allocation failed"); rc = BRT_ERR_CUDA; }
-  e->resortWords = rsWordsTotal;
+  chk(devAlloc(&e->cellPlace, n)); chk(devAlloc(&e->members, n));
+  chk(devAlloc(&e->orderCount, e->Cpad));
+  chk(devAlloc(&e->orderMem, kOrderWords + bigCellCap(e->N) + orderCellTiles(e->C)));
   if (rc) { freeAll(e); delete e; return rc; }
-  {
-    uint32_t** rsPtrs[11] = {&e->rsNewKey, &e->rsPrefix, &e->rsNext, &e->rsBlockStay, &e->rsCount, &e->rsHead,
-                             &e->rsNewStart, &e->rsTiles, &e->rsCounter, &e->rsWords, &e->rsStayBase};
-    size_t off = 0;
-    for (int k = 0; k < 11; ++k) { *rsPtrs[k] = e->resortMem + off; off += words4(rsSizes[k]); }
-  }
   e->ss = carveSortScratch(e->plan, e->sortMem, false);
   cudaStream_t st = e->stream;
   BRT_CUDA_TRY(cudaMemcpyAsync(e->flocks, e->flocksHost.data(), sizeof(FlockDev) * num_flocks, cudaMemcpyHostToDevice, st));
@@ -636,8 +606,10 @@ int brt_engine_create(const brt_params* flocks, uint32_t num_flocks, int device,
     BRT_CUDA_TRY(cudaStreamSynchronize(st));
   }
   BRT_CUDA_TRY(cudaMemsetAsync(e->sortMem, 0, sortBytes, st));
-  BRT_CUDA_TRY(resetResort(e));
+  BRT_CUDA_TRY(resetOrder(e));
   if (n) {
+    // entries of a step whose waits ran out: bounds-checked, but not undefined
+    BRT_CUDA_TRY(cudaMemsetAsync(e->members, 0xFF, n * 16, st));
     BRT_CUDA_TRY(cudaMemsetAsync(e->pairs[0], 0, n * 8, st));
     BRT_CUDA_TRY(cudaMemsetAsync(e->pairs[1], 0, n * 8, st));
   }
@@ -725,7 +697,6 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p) {
     BRT_CUDA_TRY(cudaMemcpyAsync(e->obsMask + d.cellBase, field.data() + d.cellBase, sizeof(uint2) * d.C,
                                  cudaMemcpyHostToDevice, e->stream));
   }
-  BRT_CUDA_TRY(invalidateResort(e));
   BRT_CUDA_TRY(cudaStreamSynchronize(e->stream));
   for (auto& kv : e->graphs) cudaGraphExecDestroy(kv.second);
   e->graphs.clear();
@@ -746,9 +717,8 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     if (value < 0 || value > 7) { setLastError("scan_variant must be in [0, 7]"); return BRT_ERR_ARG; }
     e->scanVariant = (int)value;
   } else if (k == "incremental_sort") {
-    e->resortOn = value != 0;
-    BRT_CUDA_TRY(invalidateResort(e));
-  } else if (k == "block_size") {
+    e->orderByCount = value != 0;
+    } else if (k == "block_size") {
     if (value < 32 || value > (int64_t)kFlockMaxThreads || value % 32) {
       setLastError("block_size must be a multiple of 32 in [32, 256]");
       return BRT_ERR_ARG;
@@ -795,8 +765,7 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     e->ss = carveSortScratch(plan, mem, false);
     e->reordered = false;
     e->listsValid = false;
-    BRT_CUDA_TRY(invalidateResort(e));
-  } else {
+    } else {
     setLastError("unknown option " + k);
     return BRT_ERR_ARG;
   }
@@ -847,11 +816,10 @@ int brt_set_state(brt_engine* e, const float* pos4, const float* fwd4, const flo
   if (e->stateLost && n) {
     // After a failed device check the slot order may hold an agent twice:
     // start again from the identity order (registered arrays included,
-    // whose contents the caller sets again) and a clean re-sort state.
+    // whose contents the caller sets again) and clean cell counts.
     BRT_CUDA_TRY(launchIota(e->idA, e->N, st));
     if (e->userIds.a) BRT_CUDA_TRY(launchIota(e->userIds.a, e->N, st));
-    // a garbled order can leave mover lists of cells that end up empty
-    BRT_CUDA_TRY(resetResort(e));
+    BRT_CUDA_TRY(resetOrder(e));
     e->stateLost = false;
   }
   auto stage4 = [&](const float* src) -> const float4* {
@@ -874,7 +842,6 @@ int brt_set_state(brt_engine* e, const float* pos4, const float* fwd4, const flo
   }
   e->reordered = false;
   e->listsValid = false;
-  BRT_CUDA_TRY(invalidateResort(e));
   if (where == BRT_MEM_HOST) BRT_CUDA_TRY(cudaStreamSynchronize(st));
   return BRT_OK;
 }
@@ -985,10 +952,8 @@ int brt_engine_stage_times(brt_engine* e, double* ms4, uint64_t* steps, uint32_t
   }
   if (ms4) for (int k = 0; k < 4; ++k) ms4[k] = e->stageMs[k];
   if (steps) *steps = e->timedSteps;
-  // hash, radix passes, reorder, flock; with the incremental re-sort also its
-  // mark, cell-scan and place kernels (the hash and the passes still launch
-  // and return at once on the steps they are not needed)
-  if (launches_per_step) *launches_per_step = 3 + e->plan.passes + (e->resortOn ? 3 : 0);
+  // count, cell scan, place, or hash and radix passes; reorder, flock
+  if (launches_per_step) *launches_per_step = 2 + (e->orderByCount ? 3 : 1 + e->plan.passes);
   e->stageMs[0] = e->stageMs[1] = e->stageMs[2] = e->stageMs[3] = 0;
   e->timedSteps = 0;
   return BRT_OK;
@@ -1027,7 +992,6 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
     } else {
       cp(e->posA, sp, n * 16); cp(e->fwdA, sf, n * 16); cp(e->accA, sa, n * 16); cp(e->statsById, ss, n * 16);
       cp(e->idA, si, n * 4); cp(e->featA, sx, n * e->Fs * 4);
-      if (c == cudaSuccess) c = invalidateResort(e);
     }
     return c;
   };
@@ -1074,16 +1038,15 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
   // single-pass kernel runs).
   uint32_t bestBits = e->plan.digitBits;
   double bestMs = 1e30, ms = 0.0;
-  // digit widths are timed with the full sort every step (the incremental
-  // re-sort would hide them)
-  const bool resortWas = e->resortOn;
-  e->resortOn = false;
+  // digit widths only matter with the radix sort
+  const bool resortWas = e->orderByCount;
+  e->orderByCount = false;
   for (uint32_t b = 4; b <= 8 && !rc; ++b) {
     chk(brt_engine_set_option(e, "sort_digit_bits", b));
     if (!rc) chk(trial("sort_digit_bits", b, &ms));
     if (!rc && ms < bestMs) { bestMs = ms; bestBits = b; }
   }
-  e->resortOn = resortWas;
+  e->orderByCount = resortWas;
   if (!rc) chk(brt_engine_set_option(e, "sort_digit_bits", bestBits));
   uint32_t bestBlock = e->fusedBlock;
   int bestScan = e->scanVariant, bestP2 = e->phase2Variant;
@@ -1141,9 +1104,9 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
     }
     if (!rc) chk(brt_engine_set_option(e, "registers", bestRegs));
   }
-  // the incremental re-sort against the full sort every step
+  // the order by counting against the radix sort
   {
-    const int start = e->resortOn ? 1 : 0;
+    const int start = e->orderByCount ? 1 : 0;
     int bestResort = start;
     bestMs = 1e30;
     for (int k = 0; k < 2 && !rc; ++k) {
@@ -1170,7 +1133,7 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
                   "{\"sort_digit_bits\": %u, \"block_size\": %u, \"scan_variant\": %d, \"phase2_variant\": %d, "
                   "\"wide_registers\": %d, \"registers\": %d, \"incremental_sort\": %d, \"ms_per_step\": %.6f, "
                   "\"trials\": [",
-                  bestBits, bestBlock, bestScan, bestP2, bestRegs > 64 ? 1 : 0, bestRegs, e->resortOn ? 1 : 0, bestMs);
+                  bestBits, bestBlock, bestScan, bestP2, bestRegs > 64 ? 1 : 0, bestRegs, e->orderByCount ? 1 : 0, bestMs);
     std::string out = std::string(buf) + log + "]}";
     std::snprintf(report, report_len, "%s", out.c_str());
   }

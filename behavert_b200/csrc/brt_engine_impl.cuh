@@ -62,17 +62,15 @@ struct brt_engine {
   void* sortMem = nullptr;
   brt::SortScratch ss;
   uint32_t* errWord = nullptr;
-  // incremental re-sort (brt_resort.cu); option "incremental_sort"
-  bool resortOn = true;
+  // the order by counting (brt_order.cu) instead of the radix sort; option "incremental_sort"
+  bool orderByCount = true;
   brt::LookbackWait wait;  // bound of the look-back waits (copied into plan.wait)
   // A device check failed (a wait ran out, a pipeline invariant broke): the
   // slot order may no longer be a permutation.  brt_set_state rebuilds it.
   bool stateLost = false;
-  uint32_t* resortMem = nullptr;   // one allocation carved into the arrays below
-  size_t resortWords = 0;          // its size in words
-  uint32_t *rsNewKey = nullptr, *rsPrefix = nullptr, *rsNext = nullptr, *rsBlockStay = nullptr;
-  uint32_t *rsCount = nullptr, *rsHead = nullptr, *rsNewStart = nullptr, *rsTiles = nullptr;
-  uint32_t *rsCounter = nullptr, *rsWords = nullptr, *rsStayBase = nullptr;
+  uint2* cellPlace = nullptr;      // OrderArgs: [N], [N], [Cpad], and words, crowded cells, scan tiles
+  uint4* members = nullptr;
+  uint32_t *orderCount = nullptr, *orderMem = nullptr;
   float4* stage4 = nullptr;  // id-order staging (N float4)
   float* stageF = nullptr;   // id-order staging (N * Fmax)
   // pipeline state
@@ -135,8 +133,6 @@ inline int devAlloc(T** p, size_t count) {
 
 // Defined in brt_engine.cu.
 int engineEnqueueStep(brt_engine* e, float dt, bool record);
-// The canonical arrays were overwritten: the next step runs the full sort.
-cudaError_t engineInvalidateResort(brt_engine* e);
 int engineSyncAndCheck(brt_engine* e);
 
 }  // namespace brt

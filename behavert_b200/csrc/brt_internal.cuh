@@ -20,10 +20,6 @@
 namespace brt {
 
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
-// Sort mode of a fused step (the incremental re-sort's decision word): the
-// hash and radix passes run only in the full-sort mode.
-constexpr uint32_t kResortFullSort = 1u, kResortIncremental = 2u;
-
 // Device error word bits (set by kernels, read by brt_engine_check_device_error).
 constexpr uint32_t kDevErrLookback = 1u;   // onesweep look-back spin limit hit
 constexpr uint32_t kDevErrCapacity = 2u;   // a per-kernel capacity check fired
@@ -125,7 +121,7 @@ __device__ __forceinline__ float imageShiftCells(int gi, int gj, uint32_t G, flo
 }
 
 // Relaxed GPU-scope load and store: the look-back words of the radix passes
-// and of the re-sort's cell scan, polled and published across CTAs.
+// and of the cell scan, polled and published across CTAs.
 __device__ __forceinline__ uint32_t ldRelaxed(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -154,10 +150,18 @@ __device__ __forceinline__ uint32_t flockOfSlot(const uint32_t* __restrict__ age
   return lo;
 }
 
+// The same, all lanes of a warp searching from its first lane's slot: the
+// loads are the warp's, and few slots then lie in a later flock.
+__device__ __forceinline__ uint32_t flockOfSlotInWarp(const uint32_t* __restrict__ agentBase, uint32_t nflocks, uint32_t slot) {
+  uint32_t f = flockOfSlot(agentBase, nflocks, slot & ~31u);
+  while (f + 1 < nflocks && __ldg(&agentBase[f + 1]) <= slot) ++f;
+  return f;
+}
+
 // ---------------------------------------------------------------------------
 // Sort plan shared by the engine and the standalone entry point.
-// Bound of every decoupled look-back wait (onesweep passes, the incremental
-// re-sort's cell scan): polls of a predecessor's unpublished status word
+// Bound of every decoupled look-back wait (onesweep passes, the cell scan
+// of the order by counting): polls of a predecessor's unpublished status word
 // before the tile gives up, records kDevErrLookback and goes on (the host
 // then reports BRT_ERR_TIMEOUT).  About a second at the default.
 // stallTile names one tile whose look-back polls as if its predecessor never
@@ -195,10 +199,8 @@ size_t sortScratchBytes(const SortPlan& p, bool withTmp);
 SortScratch carveSortScratch(const SortPlan& p, void* base, bool withTmp);
 
 // Launch one onesweep pass.
-// gate (optional): the pass runs only if *gate == kResortFullSort.
 cudaError_t launchOnesweepPass(const SortPlan& p, uint32_t pass, const uint2* in, uint2* out,
-                               const SortScratch& s, uint32_t* errWord, cudaStream_t st,
-                               const uint32_t* gate = nullptr);
+                               const SortScratch& s, uint32_t* errWord, cudaStream_t st);
 // Histogram of all passes' digits (standalone sort only; the engine fuses it
 // into the hash kernel).
 cudaError_t launchSortHistogram(const SortPlan& p, const uint2* in, const SortScratch& s, cudaStream_t st);

@@ -10,7 +10,9 @@
 //   cellStart/End    u32[C], 0xFFFFFFFF when empty;
 //   similarityStats  float4[N] in agent-id order (only the agent itself
 //                    reads it, so it never moves).
-// One step: hashKernel -> onesweep passes -> reorderKernel -> fusedKernel.
+//   members          uint4[N], the cells' agents before they are ranked by id
+// One step: the order (brt_order.cu: count, cell scan, place; or hashKernel and
+// the onesweep passes) -> reorderKernel -> flock kernel.
 #include "brt_agent.cuh"
 #include "brt_kernels.cuh"
 
@@ -27,7 +29,6 @@ namespace brt {
 // cell ranges and resets the sort's look-back state.
 __global__ void __launch_bounds__(256) hashKernel(HashArgs A) {
   extern __shared__ uint32_t sHist[];
-  if (A.gate && *A.gate != kResortFullSort) return;  // the incremental re-sort ordered this step
   const uint32_t histWords = A.passes * A.bins;
   for (uint32_t k = threadIdx.x; k < histWords; k += blockDim.x) sHist[k] = 0u;
   __syncthreads();
@@ -51,36 +52,50 @@ __global__ void __launch_bounds__(256) hashKernel(HashArgs A) {
   for (uint32_t k = gtid; k < A.statusWords; k += gstride) A.status[k] = 0u;
   if (gtid < A.passes) A.counters[gtid] = 0u;
   if (gtid == 0 && A.stepCounter) *A.stepCounter += 1u;
-  if (gtid == 0 && A.resortValid) *A.resortValid = 0u;
   __syncthreads();
   for (uint32_t k = threadIdx.x; k < histWords; k += blockDim.x)
     if (sHist[k]) atomicAdd(&A.hist[k], sHist[k]);
 }
 
 // reorderDataFloat4 (envgrid3d_kernel.cu:110-122) for every registered
-// feature in one pass with 128-bit accesses, fused with genericFindCellStartD
-// (Proximity3D_kernel.cu:54-84) extended to cellEnd.  Also clears the digit
-// histograms for the next step.
+// feature in one pass with 128-bit accesses.  After the radix sort also
+// genericFindCellStartD (Proximity3D_kernel.cu:54-84) extended to cellEnd, and
+// the clearing of the digit histograms for the next step.  RANK, after the
+// order by counting: thread i's agent is member i of its cell, in no order; its
+// sorted position is the cell's first plus the members with smaller ids (the
+// members of a cell of more than kRankLimit are in id order already).
+template <bool RANK>
 __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gstride = gridDim.x * blockDim.x;
-  for (uint32_t k = gtid; k < A.histWords; k += gstride) A.hist[k] = 0u;
-  if (A.resortMode && *A.resortMode == kResortIncremental) {
-    // the hash kernel did not clear the ranges: clear those of cells that
-    // are empty now (the others are written below)
-    for (uint32_t c = gtid; c < A.numCells; c += gstride) {
-      const uint32_t next = c + 1 < A.numCells ? A.newStart[c + 1] : A.n;
-      if (A.newStart[c] == next) { A.cellStart[c] = kEmpty; A.cellEnd[c] = kEmpty; }
-    }
-  }
-  if (gtid == 0 && A.resortValid) *A.resortValid = 1u;
+  if (!RANK)
+    for (uint32_t k = gtid; k < A.histWords; k += gstride) A.hist[k] = 0u;
   bool outside = false;  // cell-cull gate: a position of this thread's slots lies outside its cell
-  for (uint32_t i = gtid; i < A.n; i += gstride) {
-    const uint2 kv = A.pairs[i];
-    const uint32_t key = kv.x, ps = kv.y;
-    if (ps >= A.n || key >= A.numCells) { atomicOr(A.errWord, kDevErrOrder); continue; }
-    const uint32_t prev = i > 0 ? A.pairs[i - 1].x : kEmpty;
-    const uint32_t next = i + 1 < A.n ? A.pairs[i + 1].x : kEmpty;
+  for (uint32_t t = gtid; t < A.n; t += gstride) {
+    uint32_t key, ps, i = t;
+    uint32_t prev = 0, next = 0;
+    if constexpr (RANK) {
+      const uint4 m = __ldg(&A.members[t]);
+      ps = m.y;
+      key = m.w;
+      const uint32_t s = m.z;
+      // (a stale entry, left by a step whose waits ran out, must stay in bounds)
+      if (ps >= A.n || key >= A.numCells || s > t) { atomicOr(A.errWord, kDevErrOrder); continue; }
+      const uint32_t e = __ldg(&A.cellEnd[key]);
+      if (e > A.n || e <= t) { atomicOr(A.errWord, kDevErrOrder); continue; }
+      if (e - s <= kRankLimit) {
+        i = s;
+        for (uint32_t q = s; q < e; ++q) i += __ldg(&A.members[q].x) < m.x ? 1u : 0u;
+      }
+      A.pairsOut[i] = make_uint2(key, ps);
+    } else {
+      const uint2 kv = A.pairs[i];
+      key = kv.x;
+      ps = kv.y;
+      if (ps >= A.n || key >= A.numCells) { atomicOr(A.errWord, kDevErrOrder); continue; }
+      prev = i > 0 ? A.pairs[i - 1].x : kEmpty;
+      next = i + 1 < A.n ? A.pairs[i + 1].x : kEmpty;
+    }
     float4 pos = __ldg(&A.posA[ps]);
     A.fwdS[i] = __ldg(&A.fwdA[ps]);
     A.accS[i] = __ldg(&A.accA[ps]);
@@ -111,11 +126,10 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
       outside = !(pos.x >= 0.0f && pos.x <= fl.L && pos.y >= 0.0f && pos.y <= fl.L && pos.z >= 0.0f && pos.z <= fl.L);
     }
     A.posS[i] = pos;
-    if (key != prev) {
-      A.cellStart[key] = i;
-      if (A.moverHead) { A.moverHead[key] = kNoMover; A.moverCount[key] = 0u; }
+    if (!RANK) {
+      if (key != prev) A.cellStart[key] = i;
+      if (key != next) A.cellEnd[key] = i + 1;
     }
-    if (key != next) A.cellEnd[key] = i + 1;
   }
   if (A.cullWords) {
     // Scan variants 0 and 1 skip a neighbour cell by the distance from the
@@ -373,8 +387,12 @@ cudaError_t launchHash(const HashArgs& A, uint32_t smBlocks, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launchReorder(const ReorderArgs& A, cudaStream_t st) {
-  const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
-  reorderKernel<<<blocks, 256, 0, st>>>(A);
+  if (A.members) {
+    reorderKernel<true><<<std::max(1u, blocksFor(A.n, 256)), 256, 0, st>>>(A);
+  } else {
+    const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
+    reorderKernel<false><<<blocks, 256, 0, st>>>(A);
+  }
   return cudaGetLastError();
 }
 cudaError_t configureFusedKernels(uint32_t Mmax) {

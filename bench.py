@@ -836,8 +836,8 @@ def main():
     e2e_ms = max_over_ranks(pg, e2e_ms, "cuda")
     e2e_value = replica_value(world, n, E2E_HORIZON * args.e2e_iters, e2e_ms)
 
-    # the same timed runs with the full onesweep sort on every step (the
-    # incremental re-sort off), so the radix path stays measured
+    # the same timed runs with the onesweep radix sort on every step, so that
+    # path stays measured
     eng.set_option("incremental_sort", 0)
     for hs in sorted(set(horizons)):
         eng.step_prepare(dt, hs)

@@ -178,12 +178,9 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p);
    knobs, Core/src/CommonResources.cpp:78-82, generalised):
      "sort_digit_bits"  4..9  radix digit width of the onesweep passes (default 8;
                               at most 4 passes, so narrow digits on wide keys widen)
-     "incremental_sort" 0/1   derive a fused step's sorted order from the
-                              previous step's when few agents changed cell
-                              (default 1); the device falls back to the full
-                              radix sort after a state change, when more
-                              than one agent in 8 moved, or when a cell
-                              received more than 32 movers.  The order is
+     "incremental_sort" 0/1   take the sorted order by counting the agents of
+                              every cell and ranking them by id (default 1),
+                              or with the onesweep radix sort.  The order is
                               the same either way.
      "two_pass"         0/1   build each neighbour list before steering even
                               when the single-pass kernel applies (default 0)
@@ -222,7 +219,7 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p);
                               (every hash pass adds 1 before the move reads it)
      "lookback_spin_limit" 0..2^31-1: polls of an unpublished predecessor
                               before a look-back wait (onesweep passes, the
-                              re-sort's cell scan) gives up (default 2^21,
+                              order's cell scan) gives up (default 2^21,
                               about a second); the step then reports
                               BRT_ERR_TIMEOUT at the next sync or getter
      "lookback_stall_tile" -1 or a tile index: that tile's look-back polls as
@@ -283,8 +280,8 @@ int brt_step_prepare(brt_engine* e, float elapsedTime, uint32_t nsteps);
    sort, reorder and fused stages of every step.  brt_engine_stage_times
    synchronises and returns the accumulated milliseconds per stage
    (ms[0] hash, ms[1] all sort passes, ms[2] reorder + cell ranges, ms[3]
-   fused pass; with the incremental re-sort ms[0] also holds its mark kernel
-   and ms[1] its cell-scan and place kernels), the number of timed steps and
+   fused pass; with the order by counting ms[0] is its count kernel and ms[1]
+   its cell-scan and place kernels), the number of timed steps and
    the kernel launches per step. */
 int brt_engine_stage_timing(brt_engine* e, int enable);
 int brt_engine_stage_times(brt_engine* e, double* ms4, uint64_t* steps, uint32_t* launches_per_step);
@@ -388,8 +385,7 @@ int brt_engine_check_device_error(brt_engine* e, uint32_t* word);
    the registered arrays share the sorted order once a step completes.  In an
    engine with features, sorted_pos4's w holds each agent's feature norm
    (the state's pos4 keeps w = 1).  Kernels may change any value of the
-   state arrays but must not move agents between slots or rewrite agent_id:
-   the next step's incremental re-sort starts from the current slot order. */
+   state arrays but must not move agents between slots or rewrite agent_id. */
 #define BRT_MAX_USER_ARRAYS 8
 typedef struct brt_arrays {
   uint32_t num_agents, num_cells, features_stride, list_stride;
