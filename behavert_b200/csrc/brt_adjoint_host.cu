@@ -1,17 +1,19 @@
 // brt_adjoint_host.cu -- host side of the differentiable rollout (no
 // reference counterpart).
 //
-// brt_adjoint_forward runs T fused steps from the engine's current state,
-// keeping a checkpoint of the canonical state every k steps, then evaluates
-// the FP64 loss against id-ordered targets.  brt_adjoint_backward walks the
-// checkpoints from last to first: it restores one, re-runs its (up to) k
-// steps -- hash, sort, reorder and the fused pass, exactly as in the forward
-// -- with the reorder's sorted state, source slots and neighbour lists
-// written into a k-step tape, then runs the reverse kernel over the tape
-// from its last step to its first.  Both directions are captured as CUDA
-// graphs (cached by T, k, dt and the parameter version), so a whole forward
-// or backward is one graph launch.  The engine's state after the backward is
-// the final state of the forward.
+// brt_adjoint_forward runs T fused steps from the engine's current state, then
+// evaluates the FP64 loss against id-ordered targets.  The reverse kernels read
+// a tape: every step's sorted state, source slots and neighbour lists.  Where
+// the tape of all T steps fits (wholeTapeFits), the forward's steps write
+// straight into it and brt_adjoint_backward runs the reverse kernels from the
+// last step to the first.  Otherwise the forward keeps a checkpoint of the
+// canonical state every k steps, and the backward walks the checkpoints from
+// last to first: it restores one, re-runs its (up to) k steps -- order, reorder
+// and the fused pass, exactly as in the forward -- into a k-step tape, and runs
+// the reverse kernels over that.  Both directions are captured as CUDA graphs
+// (cached by T, k, dt and the parameter version), so a whole forward or
+// backward is one graph launch.  The engine's state after the backward is the
+// final state of the forward.
 #include "brt_engine_impl.cuh"
 
 #include <cstring>
@@ -27,7 +29,8 @@ struct AdjointState {
   bool taped = false;
   uint32_t version = 0;       // engine paramsVersion of the taped forward
   uint32_t weightsVersion = 0;
-  uint32_t capCk = 0, capK = 0, capExport = 0;
+  bool whole = false;         // tape[0] holds all T steps of the forward (wholeTapeFits)
+  uint32_t capCk = 0, capK[2] = {0, 0}, capExport = 0;
   std::vector<void*> mem;
   // checkpoints (nck x N) and the saved final state
   float4 *ckPos = nullptr, *ckFwd = nullptr, *ckAcc = nullptr;
@@ -105,9 +108,28 @@ int checkSupported(brt_engine* e) {
   return BRT_OK;
 }
 
+// Whether the forward keeps every step's sorted state and lists instead of
+// checkpoints, so that the backward has nothing to compute again: when they
+// take at most an eighth of the device's memory, and at most half of what is
+// free beside the tape's present size.  Measured with the recompute beside the
+// reverse on a second stream / without it: 65,536 agents x 50 steps (0.4 GB)
+// 8.9 / 6.9 ms forward and backward, 64 flocks of 499 k agents x 40 (2.5 GB)
+// 39.0 / 31.0 ms.
+bool wholeTapeFits(brt_engine* e, uint32_t T) {
+  if (e->adjointCheckpoints) return false;
+  if (T <= e->adj->capK[0]) return true;  // there already
+  const size_t step = (size_t)e->N * (3 * 16 + 2 * 4 + 4 * (size_t)e->listStride);
+  size_t freeBytes = 0, total = 0;
+  if (cudaMemGetInfo(&freeBytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return step * T <= total / 8 && step * T <= (freeBytes + step * e->adj->capK[0]) / 2;
+}
+
 // (Re)allocates the checkpoint and tape storage for nck checkpoints and k
-// tape steps; buffers only grow.
-int ensureCapacity(brt_engine* e, uint32_t nck, uint32_t k, uint32_t T) {
+// tape steps (whole: one tape of T steps); buffers only grow.
+int ensureCapacity(brt_engine* e, uint32_t nck, uint32_t k, uint32_t T, bool whole) {
   AdjointState* a = e->adj;
   const size_t n = e->N;
   int rc = BRT_OK;
@@ -155,14 +177,18 @@ int ensureCapacity(brt_engine* e, uint32_t nck, uint32_t k, uint32_t T) {
     a->capCk = nck;
     changed = true;
   }
-  if (k > a->capK) {
+  for (int i = 0; i < (whole ? 1 : 2); ++i) {
+    if (k <= a->capK[i]) continue;
     BRT_CUDA_TRY(cudaStreamSynchronize(e->stream));
-    for (auto& t : a->tape)
-      if ((rc = regrow(&t.pos, n * k)) || (rc = regrow(&t.fwd, n * k)) || (rc = regrow(&t.acc, n * k)) ||
-          (rc = regrow(&t.prev, n * k)) || (rc = regrow(&t.id, n * k)) || (rc = regrow(&t.lists, n * k * e->listStride)))
-        return rc;
-    a->capK = k;
+    AdjointState::Tape& t = a->tape[i];
+    a->capK[i] = 0;
     changed = true;
+    if ((rc = regrow(&t.pos, n * k)) || (rc = regrow(&t.fwd, n * k)) || (rc = regrow(&t.acc, n * k)) ||
+        (rc = regrow(&t.prev, n * k)) || (rc = regrow(&t.id, n * k)) || (rc = regrow(&t.lists, n * k * e->listStride))) {
+      dropGraphs(a);
+      return rc;
+    }
+    a->capK[i] = k;
   }
   if (!a->revStream) BRT_CUDA_TRY(cudaStreamCreateWithFlags(&a->revStream, cudaStreamNonBlocking));
   while (a->events.size() < 2 * (size_t)nck) {
@@ -193,6 +219,31 @@ int copyState(brt_engine* e, float4* pos, float4* fwd, float4* acc, uint32_t* id
   return BRT_OK;
 }
 
+// Runs steps with a tape as their sorted-state and list buffers: the forward's
+// (whole tape), or one segment's again.
+int enqueueTaped(brt_engine* e, uint32_t steps, const AdjointState::Tape& tp, bool again) {
+  AdjointState* a = e->adj;
+  const size_t n = e->N;
+  float4 *posS = e->posS, *fwdS = e->fwdS, *accS = e->accS;
+  uint32_t *idS = e->idS, *lists = e->lists;
+  // after a segment's recompute the engine returns to the forward's final
+  // state, so registered arrays (already at that state) are not permuted again
+  const bool wasFrozen = e->userFrozen;
+  e->userFrozen = wasFrozen || again;
+  int rc = BRT_OK;
+  for (uint32_t s = 0; s < steps && !rc; ++s) {
+    e->posS = tp.pos + s * n; e->fwdS = tp.fwd + s * n; e->accS = tp.acc + s * n;
+    e->idS = tp.id + s * n;
+    e->lists = tp.lists + s * n * e->listStride;
+    e->tapePrev = tp.prev + s * n;
+    rc = engineEnqueueStep(e, a->dt, true);
+  }
+  e->posS = posS; e->fwdS = fwdS; e->accS = accS; e->idS = idS; e->lists = lists;
+  e->tapePrev = nullptr;
+  e->userFrozen = wasFrozen;
+  return rc;
+}
+
 // The taped forward: checkpoints, steps, final state, loss.
 int enqueueForward(brt_engine* e) {
   AdjointState* a = e->adj;
@@ -203,6 +254,10 @@ int enqueueForward(brt_engine* e) {
                         e->accA, e->idA)))
       return rc;
     const uint32_t steps = std::min(a->k, a->T - c * a->k);
+    if (a->whole) {
+      if ((rc = enqueueTaped(e, steps, a->tape[0], false))) return rc;
+      continue;
+    }
     for (uint32_t s = 0; s < steps; ++s)
       if ((rc = engineEnqueueStep(e, a->dt, false))) return rc;
   }
@@ -219,31 +274,6 @@ int enqueueForward(brt_engine* e) {
   R.partial = a->partial;
   BRT_CUDA_TRY(launchFlockReduce(R, e->stream));
   return BRT_OK;
-}
-
-// Re-runs one segment's steps with a tape as the step's sorted-state and
-// list buffers.
-int enqueueRecompute(brt_engine* e, uint32_t steps, const AdjointState::Tape& tp) {
-  AdjointState* a = e->adj;
-  const size_t n = e->N;
-  float4 *posS = e->posS, *fwdS = e->fwdS, *accS = e->accS;
-  uint32_t *idS = e->idS, *lists = e->lists;
-  // the engine returns to the forward's final state afterwards, so
-  // registered arrays (already at that state) are not permuted again
-  const bool wasFrozen = e->userFrozen;
-  e->userFrozen = true;
-  int rc = BRT_OK;
-  for (uint32_t s = 0; s < steps && !rc; ++s) {
-    e->posS = tp.pos + s * n; e->fwdS = tp.fwd + s * n; e->accS = tp.acc + s * n;
-    e->idS = tp.id + s * n;
-    e->lists = tp.lists + s * n * e->listStride;
-    e->tapePrev = tp.prev + s * n;
-    rc = engineEnqueueStep(e, a->dt, true);
-  }
-  e->posS = posS; e->fwdS = fwdS; e->accS = accS; e->idS = idS; e->lists = lists;
-  e->tapePrev = nullptr;
-  e->userFrozen = wasFrozen;
-  return rc;
 }
 
 // variant bits: 1 extra position adjoint, 2 extra forward adjoint, 4 extra
@@ -272,8 +302,10 @@ int enqueueBackward(brt_engine* e, uint32_t variant) {
   // beside it into the other tape, once the reverse of c + 1 (the last
   // reader of that tape) is done.  Both are latency-bound at these sizes, so
   // the two overlap on the GPU; the results are those of running them in
-  // sequence.
-  cudaStream_t rs = a->revStream;
+  // sequence.  A whole tape has no recompute: the reverse runs on the engine
+  // stream.
+  const bool whole = a->whole;
+  cudaStream_t rs = whole ? e->stream : a->revStream;
   auto evRecomputed = [a](int c) { return a->events[2 * (size_t)c]; };
   auto evReversed = [a](int c) { return a->events[2 * (size_t)c + 1]; };
   auto recompute = [&](int c) -> int {
@@ -282,13 +314,13 @@ int enqueueBackward(brt_engine* e, uint32_t variant) {
                       a->ckId + c * n);
     if (r) return r;
     const uint32_t steps = std::min(a->k, a->T - (uint32_t)c * a->k);
-    if ((r = enqueueRecompute(e, steps, a->tape[c & 1]))) return r;
+    if ((r = enqueueTaped(e, steps, a->tape[c & 1], true))) return r;
     BRT_CUDA_TRY(cudaEventRecord(evRecomputed(c), e->stream));
     return BRT_OK;
   };
-  if ((rc = recompute((int)a->nck - 1))) return rc;
+  if (!whole && (rc = recompute((int)a->nck - 1))) return rc;
   for (int c = (int)a->nck - 1; c >= 0; --c) {
-    BRT_CUDA_TRY(cudaStreamWaitEvent(rs, evRecomputed(c), 0));
+    if (!whole) BRT_CUDA_TRY(cudaStreamWaitEvent(rs, evRecomputed(c), 0));
     const AdjointState::Tape& tp = a->tape[c & 1];
     const uint32_t steps = std::min(a->k, a->T - (uint32_t)c * a->k);
     for (int s = (int)steps - 1; s >= 0; --s) {
@@ -314,10 +346,11 @@ int enqueueBackward(brt_engine* e, uint32_t variant) {
       BRT_CUDA_TRY(launchAdjointStep(R, rs));
       cur ^= 1;
     }
+    if (whole) break;  // one segment, on the engine stream
     BRT_CUDA_TRY(cudaEventRecord(evReversed(c), rs));
     if (c > 0 && (rc = recompute(c - 1))) return rc;
   }
-  BRT_CUDA_TRY(cudaStreamWaitEvent(e->stream, evReversed(0), 0));
+  if (!whole) BRT_CUDA_TRY(cudaStreamWaitEvent(e->stream, evReversed(0), 0));
   FlockReduceArgs W;
   W.vals = a->accW; W.width = 3; W.agentBase = e->agentBase; W.nflocks = e->nflocks; W.out = a->gW;
   W.partial = a->partial;
@@ -398,10 +431,17 @@ int brt_adjoint_forward(brt_engine* e, float elapsedTime, uint32_t nsteps, uint3
   DeviceGuard guard(e->device);
   if (!e->adj) e->adj = new AdjointState();
   AdjointState* a = e->adj;
-  const uint32_t k = std::min(checkpoint_every, nsteps);
+  if ((rc = ensureCapacity(e, 1, 0, nsteps, true))) return rc;  // everything but the tape
+  bool whole = wholeTapeFits(e, nsteps);
+  if (whole && ensureCapacity(e, 1, nsteps, nsteps, true)) {
+    cudaGetLastError();  // the memory went to someone else meanwhile: checkpoints
+    whole = false;
+  }
+  const uint32_t k = whole ? nsteps : std::min(checkpoint_every, nsteps);
   const uint32_t nck = (nsteps + k - 1) / k;
-  if ((rc = ensureCapacity(e, nck, k, nsteps))) return rc;
-  if (a->T != nsteps || a->k != k || a->dt != elapsedTime) dropGraphs(a);
+  if (!whole && (rc = ensureCapacity(e, nck, k, nsteps, false))) return rc;
+  if (a->T != nsteps || a->k != k || a->dt != elapsedTime || a->whole != whole) dropGraphs(a);
+  a->whole = whole;
   a->T = nsteps; a->k = k; a->nck = nck; a->dt = elapsedTime;
   a->taped = false;
   BRT_CUDA_TRY(cudaMemcpyAsync(a->target, target_pos4, (size_t)e->N * 16, kindIn(where), e->stream));

@@ -742,6 +742,8 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     e->adjointGraphs = value != 0;
   } else if (k == "adjoint_export") {
     e->adjointExport = value != 0;
+  } else if (k == "adjoint_checkpoints") {
+    e->adjointCheckpoints = value != 0;
   } else if (k == "lookback_spin_limit") {
     if (value < 0 || value > 0x7FFFFFFFll) { setLastError("lookback_spin_limit must be in [0, 2^31)"); return BRT_ERR_ARG; }
     e->wait.spinLimit = (uint32_t)value;

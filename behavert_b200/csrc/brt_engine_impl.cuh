@@ -92,6 +92,7 @@ struct brt_engine {
   brt::AdjointState* adj = nullptr;
   bool adjointGraphs = true;  // option "adjoint_graphs"
   bool adjointExport = false; // option "adjoint_export"
+  bool adjointCheckpoints = false; // option "adjoint_checkpoints"
   uint32_t weightsVersion = 0; // bumped by brt_set_steering_weights
   // registered per-agent arrays (brt_engine_add_array): `a` holds the array in
   // the engine's slot order, `s` is the gather target of each reorder (copied

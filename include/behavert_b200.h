@@ -214,6 +214,11 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p);
                               a thread (64 default; 48 and 40 trade spills for
                               resident warps and apply to scan_variant 4, 5, 7)
      "adjoint_graphs"   0/1   capture the adjoint forward/backward as graphs (default 1)
+     "adjoint_checkpoints" 0/1  1: brt_adjoint_forward always keeps checkpoints
+                              and the backward computes their segments again;
+                              0 (default): it keeps every step's tape where
+                              that takes at most an eighth of the device's
+                              memory and half of what is free
      "adjoint_export"   0/1   keep the frozen lists and branch flags (brt_adjoint_get_tape)
      "random_step"      uint32 the step counter of the Schooling random stream
                               (every hash pass adds 1 before the move reads it)
@@ -418,7 +423,8 @@ int brt_engine_launch(brt_engine* e, brt_launch_fn fn, void* user_data);
    steering and maxNeighbors > 32 return BRT_ERR_CONFIG.
 
    brt_adjoint_forward runs nsteps fused steps from the current state,
-   checkpointing the state every checkpoint_every steps, and evaluates
+   checkpointing the state every checkpoint_every steps (or keeping the tape of
+   every step, where it fits: option "adjoint_checkpoints"), and evaluates
        loss_f = (1 / n_f) sum_{i in flock f} |minimum image(p_i(T) - target_i)|^2
    in FP64 (target_pos4: float4 per agent in agent-id order).  loss_per_flock
    (nflocks doubles, may be NULL) follows `where`.  The engine is left at the
@@ -427,8 +433,8 @@ int brt_engine_launch(brt_engine* e, brt_launch_fn fn, void* user_data);
    brt_adjoint_backward propagates the adjoint of
        sum_f loss_scale[f] * loss_f  (+ <g*_T, final state> for the optional
        id-ordered adjoints gpos4_T / gfwd4_T (xyz forward, w speed) / gacc4_T)
-   back through the taped forward, recomputing hash, sort and neighbour lists
-   of each checkpoint segment.  loss_scale: host array of nflocks doubles or
+   back through the taped forward, recomputing the order and neighbour lists
+   of each checkpoint segment (unless the forward kept them).  loss_scale: host array of nflocks doubles or
    NULL for 1.  Outputs (float4 per agent, agent-id order, each may be NULL):
    grad_pos4 = dL/dposition(0), grad_fwd4 = dL/dforward(0) (w = dL/dspeed),
    grad_vel4 = dL/dvelocity(0) with velocity = forward * speed,
