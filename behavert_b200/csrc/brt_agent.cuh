@@ -322,26 +322,51 @@ __device__ __forceinline__ float fromOrderedBits(uint32_t u) {
 // s_{k+1} = max(list) and the next one is at most max(s_{k+1}, d) <
 // max(s_{k+1}, s_k).  A candidate at or beyond B = max(s, previous s) can
 // never replace an entry and is skipped before the serial replacements.
-// The first M accepted go in with one ballot, as in the first-M scan.
-template <int R, int WINT = 0, bool CULL = false, bool KNN = false>
-__device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32_t self, f3 p, uint32_t key,
+// The first M accepted go in with one ballot, as in the first-M scan.  Once a
+// list is full its ceiling B shrinks, and in a crowded cell most rounds hold no
+// candidate below it: a vote on the squared distances leaves those rounds, and
+// windows without any, before the square roots (a window's ceiling at its start
+// is never below a later one).
+//
+// Each run's segments (the non-empty ones of the 27 cells) are laid out in
+// shared memory (segs, kSegments per warp), or with SEGREG in registers (the k-th
+// in lane k), where that memory would cost a resident block; a round finds its candidates'
+// segments by counting the segment starts among its 32 positions (one warp-wide
+// OR and a population count) instead of searching the 27 prefixes with five
+// dependent shuffles and five more for the found segment's data.  With the
+// flock's parameters kept from run to run that took a third of the setup's
+// instructions out.
+constexpr uint32_t kSegments = 27;
+// An agent's home cell: the global cell key, and the three coordinates in ten
+// bits each (an engine has at most 2^30 cells).
+struct HomeCell {
+  uint32_t key, at;
+};
+__device__ __forceinline__ HomeCell homeCell(int gx, int gy, int gz, const FlockDev& fl) {
+  return {fl.cellBase + ((uint32_t)gz * fl.G + (uint32_t)gy) * fl.G + (uint32_t)gx,
+          (uint32_t)gx | (uint32_t)gy << 10 | (uint32_t)gz << 20};
+}
+template <int R, int WINT = 0, bool CULL = false, bool KNN = false, bool SEGREG = false>
+__device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32_t self, f3 p, HomeCell home,
                                                              const FlockDev* __restrict__ flocks, uint32_t flock,
                                                              const uint32_t* __restrict__ cellStart,
                                                              const uint32_t* __restrict__ cellEnd,
                                                              const float4* __restrict__ posS, uint32_t* sList,
-                                                             uint32_t ls, uint32_t laneCol0, float4* cbuf = nullptr,
-                                                             float* dList = nullptr) {
+                                                             uint32_t ls, uint32_t laneCol0, float4* segs,
+                                                             float4* cbuf = nullptr, float* dList = nullptr) {
   static_assert(!CULL || R > 0, "the culled scan votes on register-held rounds");
   static_assert(!KNN || (R > 0 && !CULL), "the kNN scan votes on register-held rounds, unculled");
   const uint32_t full = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t myKey = active ? key : 0xFFFFFFFFu;
+  const uint32_t myKey = active ? home.key : 0xFFFFFFFFu;
   const uint32_t prevKey = __shfl_up_sync(full, myKey, 1);
   const bool head = active && (lane == 0 || prevKey != myKey);
   uint32_t heads = __ballot_sync(full, head);
   const uint32_t activeMask = __ballot_sync(full, active);
   uint32_t n = 0;
-  float kmx = 0.0f, kmxPrev = 0.0f;  // kNN: the lane's agent's bound (maxDistValue) and its previous value
+  // kNN: the lane's agent's bound (maxDistValue), its previous value, and a
+  // squared distance above which a candidate cannot enter the list
+  float kmx = 0.0f, kmxPrev = 0.0f, kB2 = 0.0f;
   // bounding box of the lane's run: lanes of equal key (a run, or with a
   // corrupted order a superset of it, which only culls less)
   float bLo[3] = {0.f, 0.f, 0.f}, bHi[3] = {0.f, 0.f, 0.f};
@@ -362,6 +387,12 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
       bHi[0] = bHi[1] = bHi[2] = INFINITY;
     }
   }
+  // this lane's neighbour cell (lanes 0..26, in visit order), and the
+  // parameters of the flock at hand (a warp's agents are mostly of one)
+  const int ox = (int)(lane / 9u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane % 3u) - 1;
+  const uint32_t belowLane = (1u << lane) - 1u;
+  uint32_t held = 0xFFFFFFFFu, M = 0, G = 0, cellBase = 0, slotLo = 0, slotHi = 0, most = 0;
+  float thr = 0.0f, L = 0.0f;
   while (heads) {
     const uint32_t g0 = __ffs(heads) - 1;
     heads &= heads - 1;
@@ -370,28 +401,34 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
     const uint32_t groupMask = activeMask & (((g1 >= 32u) ? full : ((1u << g1) - 1u)) & ~((1u << g0) - 1u));
     const uint32_t f = __shfl_sync(full, flock, g0);
     const FlockDev& fl = flocks[f];
-    const uint32_t M = fl.M;
-    const float thr = fl.r2thr;
-    const uint32_t G = fl.G;
+    if (f != held) {
+      held = f;
+      M = fl.M;
+      thr = fl.r2thr;
+      G = fl.G;
+      L = fl.L;
+      cellBase = fl.cellBase;
+      slotLo = fl.agentBase;
+      slotHi = slotLo + fl.n;
+      most = fl.maxPerCell ? fl.maxPerCell : 0xFFFFFFFFu;
+    }
     // home cell coordinates from the group's first agent
-    const float px = __shfl_sync(full, p.x, g0), py = __shfl_sync(full, p.y, g0), pz = __shfl_sync(full, p.z, g0);
-    const int gx = gridCoord(px, fl), gy = gridCoord(py, fl), gz = gridCoord(pz, fl);
+    const uint32_t at = __shfl_sync(full, home.at, g0);
+    const int gx = (int)(at & 1023u), gy = (int)(at >> 10 & 1023u), gz = (int)(at >> 20);
     // lanes 0..26: one neighbour cell each, in visit order
     uint32_t segStart = 0, segLen = 0;
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     if (lane < 27u) {
-      const int ox = (int)(lane / 9u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane % 3u) - 1;
       const int cx = wrapCoord(gx + ox, G), cy = wrapCoord(gy + oy, G), cz = wrapCoord(gz + oz, G);
-      const uint32_t h = fl.cellBase + ((uint32_t)cz * G + (uint32_t)cy) * G + (uint32_t)cx;
+      const uint32_t h = cellBase + ((uint32_t)cz * G + (uint32_t)cy) * G + (uint32_t)cx;
       const uint32_t st = __ldg(&cellStart[h]), en = __ldg(&cellEnd[h]);
-      if (usableRange(fl, st, en)) {
+      if (st < en && st >= slotLo && en <= slotHi) {  // usableRange
         segStart = st;
-        segLen = en - st;
-        if (fl.maxPerCell && segLen > fl.maxPerCell) segLen = fl.maxPerCell;
+        segLen = min(en - st, most);
       }
-      sx = imageShift(gx, ox, G, fl.L);
-      sy = imageShift(gy, oy, G, fl.L);
-      sz = imageShift(gz, oz, G, fl.L);
+      sx = imageShift(gx, ox, G, L);
+      sy = imageShift(gy, oy, G, L);
+      sz = imageShift(gz, oz, G, L);
     }
     // exclusive prefix of the segment lengths
     uint32_t incl = segLen;
@@ -402,12 +439,41 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
     }
     const uint32_t excl = incl - segLen;
     const uint32_t total = __shfl_sync(full, incl, 31);
+    // the segments that are not empty, one after the other: slot of candidate
+    // t is delta + t
+    const bool some = segLen != 0u;
+    const uint32_t nonEmpty = __ballot_sync(full, some);
+    float4 seg0 = make_float4(__uint_as_float(segStart - excl), sx, sy, sz);
+    if constexpr (SEGREG) {
+      const uint32_t from = nthSetBit(nonEmpty, lane) & 31u;
+      seg0 = make_float4(__shfl_sync(full, seg0.x, from), __shfl_sync(full, seg0.y, from), __shfl_sync(full, seg0.z, from),
+                         __shfl_sync(full, seg0.w, from));
+    } else {
+      __syncwarp();  // every lane is done with the previous run's
+      if (some) segs[__popc(nonEmpty & belowLane)] = seg0;
+      __syncwarp();
+    }
+    // The segment of candidate base + lane (base a multiple of 32, below
+    // total): one more than the segments that start before base, counted on
+    // from the ones that start at base .. base + lane.
+    auto segmentOf = [&](uint32_t base) -> float4 {
+      const uint32_t rel = excl - base;
+      const uint32_t starts = __reduce_or_sync(full, some && rel < 32u ? 1u << rel : 0u);
+      const uint32_t earlier = (uint32_t)__popc(__ballot_sync(full, some && excl < base));
+      const uint32_t k = earlier + (uint32_t)__popc(starts & (belowLane * 2u + 1u)) - 1u;
+      if constexpr (SEGREG)
+        return make_float4(__shfl_sync(full, seg0.x, k), __shfl_sync(full, seg0.y, k), __shfl_sync(full, seg0.z, k),
+                           __shfl_sync(full, seg0.w, k));
+      else
+        return segs[k];
+    };
     uint32_t open = groupMask;  // group agents whose list is not full yet
     uint32_t base0 = 0;
     if constexpr (KNN) {
       if (fl.useKnn) {
         constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
         const float radius = fl.radius;
+        if (groupMask >> lane & 1u) kB2 = thr;
         for (; base0 < total; base0 += (uint32_t)R * 32u) {
           float cqx[R], cqy[R], cqz[R];
           uint32_t cslot[R];
@@ -417,27 +483,30 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
             cslot[r] = kNoSlot;
             if (base0 + (uint32_t)r * 32u < total) {
               const uint32_t t = base0 + (uint32_t)r * 32u + lane;
-              uint32_t c = 0;
-#pragma unroll
-              for (int step = 16; step > 0; step >>= 1) {
-                const uint32_t cand = c + (uint32_t)step;
-                const uint32_t e = __shfl_sync(full, excl, cand & 31u);
-                if (cand < 27u && e <= t) c = cand;
-              }
-              const uint32_t cStart = __shfl_sync(full, segStart, c), cExcl = __shfl_sync(full, excl, c);
-              const float csx = __shfl_sync(full, sx, c), csy = __shfl_sync(full, sy, c), csz = __shfl_sync(full, sz, c);
+              const float4 seg = segmentOf(base0 + (uint32_t)r * 32u);
               if (t < total) {
-                cslot[r] = cStart + (t - cExcl);
+                cslot[r] = __float_as_uint(seg.x) + t;
                 const float4 q = __ldg(&posS[cslot[r]]);
-                cqx[r] = q.x + csx;
-                cqy[r] = q.y + csy;
-                cqz[r] = q.z + csz;
+                cqx[r] = q.x + seg.y;
+                cqy[r] = q.y + seg.z;
+                cqz[r] = q.z + seg.w;
               }
             }
           }
           for (uint32_t todo = groupMask; todo; todo &= todo - 1u) {
             const uint32_t a = __ffs(todo) - 1u;
             const float ax = __shfl_sync(full, p.x, a), ay = __shfl_sync(full, p.y, a), az = __shfl_sync(full, p.z, a);
+            // a window without a candidate inside the agent's bound changes nothing
+            const float aB2 = __shfl_sync(full, kB2, a);
+            float d2[R];
+            bool near = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float dx = cqx[r] - ax, dy = cqy[r] - ay, dz = cqz[r] - az;
+              d2[r] = dx * dx + dy * dy + dz * dz;
+              near = near || (cslot[r] != kNoSlot && !(d2[r] > aB2));
+            }
+            if (!__any_sync(full, near)) continue;
             const uint32_t aSelf = __shfl_sync(full, self, a);
             uint32_t an = __shfl_sync(full, n, a);
             float amx = __shfl_sync(full, kmx, a), amxPrev = __shfl_sync(full, kmxPrev, a);
@@ -453,9 +522,8 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
             }
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              if (base0 + (uint32_t)r * 32u >= total) break;
-              const float dx = cqx[r] - ax, dy = cqy[r] - ay, dz = cqz[r] - az;
-              const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
+              if (!__any_sync(full, cslot[r] != kNoSlot && !(d2[r] > aB2))) continue;
+              const float dist = sqrtf(d2[r]);
               const bool acc = cslot[r] != kNoSlot && cslot[r] != aSelf && !(dist > radius);
               uint32_t bal = __ballot_sync(full, acc);
               if (an < M) {
@@ -513,7 +581,16 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
               col[lane * ls] = ks;
               dcol[lane * ls] = kd;
             }
-            if (lane == a) { n = an; kmx = amx; kmxPrev = amxPrev; }
+            if (lane == a) {
+              n = an;
+              kmx = amx;
+              kmxPrev = amxPrev;
+              if (an == M) {
+                // dist < ceiling only where d2 is below its square (a little above, for the roundings)
+                const float ceilB = fmaxf(amx, amxPrev);
+                kB2 = fminf(thr, ceilB * ceilB * 1.000001f + 1e-44f);
+              }
+            }
           }
         }
         continue;  // the next run
@@ -531,21 +608,13 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
         // R * 32 - 1 + 32 entries: the buffer holds (R + 1) * 32)
         while (buffered < (uint32_t)R * 32u && raw < total) {
           const uint32_t t = raw + lane;
-          uint32_t c = 0;
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1) {
-            const uint32_t cand = c + (uint32_t)step;
-            const uint32_t e = __shfl_sync(full, excl, cand & 31u);
-            if (cand < 27u && e <= t) c = cand;
-          }
-          const uint32_t cStart = __shfl_sync(full, segStart, c), cExcl = __shfl_sync(full, excl, c);
-          const float csx = __shfl_sync(full, sx, c), csy = __shfl_sync(full, sy, c), csz = __shfl_sync(full, sz, c);
+          const float4 seg = segmentOf(raw);
           bool keep = false;
           float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
           if (t < total) {
-            const uint32_t slot = cStart + (t - cExcl);
+            const uint32_t slot = __float_as_uint(seg.x) + t;
             const float4 q = __ldg(&posS[slot]);
-            v = make_float4(q.x + csx, q.y + csy, q.z + csz, __uint_as_float(slot));
+            v = make_float4(q.x + seg.y, q.y + seg.z, q.z + seg.w, __uint_as_float(slot));
             const float ex = fmaxf(fmaxf(lx - v.x, v.x - hx), 0.0f);
             const float ey = fmaxf(fmaxf(ly - v.y, v.y - hy), 0.0f);
             const float ez = fmaxf(fmaxf(lz - v.z, v.z - hz), 0.0f);
@@ -624,21 +693,13 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
           cslot[r] = kNoSlot;
           if (base0 + (uint32_t)r * 32u < total) {
             const uint32_t t = base0 + (uint32_t)r * 32u + lane;
-            uint32_t c = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-              const uint32_t cand = c + (uint32_t)step;
-              const uint32_t e = __shfl_sync(full, excl, cand & 31u);
-              if (cand < 27u && e <= t) c = cand;
-            }
-            const uint32_t cStart = __shfl_sync(full, segStart, c), cExcl = __shfl_sync(full, excl, c);
-            const float csx = __shfl_sync(full, sx, c), csy = __shfl_sync(full, sy, c), csz = __shfl_sync(full, sz, c);
+            const float4 seg = segmentOf(base0 + (uint32_t)r * 32u);
             if (t < total) {
-              cslot[r] = cStart + (t - cExcl);
+              cslot[r] = __float_as_uint(seg.x) + t;
               const float4 q = __ldg(&posS[cslot[r]]);
-              cqx[r] = q.x + csx;
-              cqy[r] = q.y + csy;
-              cqz[r] = q.z + csz;
+              cqx[r] = q.x + seg.y;
+              cqy[r] = q.y + seg.z;
+              cqz[r] = q.z + seg.w;
             }
           }
         }
@@ -673,19 +734,10 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
     for (uint32_t base = base0; base < total && open; base += 32u) {
       const uint32_t t = base + lane;
       const bool valid = t < total;
-      // segment of t: the last segment whose exclusive prefix is <= t
-      uint32_t c = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const uint32_t cand = c + (uint32_t)step;
-        const uint32_t e = __shfl_sync(full, excl, cand & 31u);
-        if (cand < 27u && e <= t) c = cand;
-      }
-      const uint32_t cStart = __shfl_sync(full, segStart, c), cExcl = __shfl_sync(full, excl, c);
-      const float csx = __shfl_sync(full, sx, c), csy = __shfl_sync(full, sy, c), csz = __shfl_sync(full, sz, c);
-      const uint32_t slot = valid ? cStart + (t - cExcl) : 0xFFFFFFFFu;
+      const float4 seg = segmentOf(base);
+      const uint32_t slot = valid ? __float_as_uint(seg.x) + t : 0xFFFFFFFFu;
       const float4 q = valid ? __ldg(&posS[slot]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float qx = q.x + csx, qy = q.y + csy, qz = q.z + csz;
+      const float qx = q.x + seg.y, qy = q.y + seg.z, qz = q.z + seg.w;
       for (uint32_t todo = open; todo; todo &= todo - 1u) {
         const uint32_t a = __ffs(todo) - 1u;
         const float ax = __shfl_sync(full, p.x, a), ay = __shfl_sync(full, p.y, a), az = __shfl_sync(full, p.z, a);

@@ -355,7 +355,8 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   // kNN flocks take its cooperative kNN scan (scan 8).
   bool twoPass = e->forceTwoPass || (e->anyKnn && e->Mmax > 32);
   for (const FlockDev& d : e->flocksHost) twoPass = twoPass || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
-  if (e->anyKnn && !twoPass) F.scanVariant = 8;
+  if (e->anyKnn && !twoPass) F.scanVariant = flockKnnScan(e->fusedBlock, e->Mmax, e->regBudget);
+  F.taped = e->tapePrev != nullptr;
   F.warpAgents = e->school ? e->schoolWarp
                  : twoPass ? e->fusedWarp
                            : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);

@@ -40,10 +40,12 @@ constexpr uint32_t kCullBufPerWarp = (kCoopCachedRounds + 1) * 32;
 __host__ __device__ constexpr uint32_t cullBufOffsetWords(uint32_t ls, uint32_t Mmax) { return (ls * Mmax + 3u) & ~3u; }
 // Scan 8 (the cooperative scan with the kNN replacement, for engines with a
 // useKnn flock and maxNeighbors <= 32) keeps each list's distances beside it.
+// The cooperative scans' run segments come first (kSegments per warp).
 __host__ __device__ constexpr size_t flockSmemBytes(uint32_t block, uint32_t Mmax, int scan) {
-  return scan == 7   ? (size_t)cullBufOffsetWords(block + 1, Mmax) * 4 + (size_t)(block / 32) * kCullBufPerWarp * 16
-         : scan == 8 ? (size_t)2 * (block + 1) * Mmax * 4
-                     : (size_t)(block + (scan >= 4 ? 1u : 0u)) * Mmax * 4;
+  return (scan >= 4 && scan != 9 ? (size_t)(block / 32) * kSegments * 16 : 0) +
+         (scan == 7   ? (size_t)cullBufOffsetWords(block + 1, Mmax) * 4 + (size_t)(block / 32) * kCullBufPerWarp * 16
+         : scan >= 8 ? (size_t)2 * (block + 1) * Mmax * 4
+                     : (size_t)(block + (scan >= 4 ? 1u : 0u)) * Mmax * 4);
 }
 
 // Phase 2 of the flock kernels: steering and feature sums over agent i's
@@ -224,7 +226,8 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
 
 template <int FP, int P2, int MINB, int SCAN>
 __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs A) {
-  extern __shared__ __align__(16) uint32_t sList[];
+  extern __shared__ __align__(16) uint32_t sFlock[];
+  uint32_t* sList = sFlock + (SCAN >= 4 && SCAN != 9 ? (blockDim.x >> 5) * kSegments * 4u : 0u);
   // The warp-cooperative scans need every lane of the warp; inactive lanes
   // take part read-only (mirroring the last agent) and leave after it.
   constexpr bool coop = SCAN != 0;
@@ -253,18 +256,19 @@ __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs 
   (void)M;
   uint32_t n;
   if (SCAN >= 4) {
-    const uint32_t key = fl.cellBase + ((uint32_t)gz * G + (uint32_t)gy) * G + (uint32_t)gx;
+    const HomeCell key = homeCell(gx, gy, gz, fl);
+    float4* segs = reinterpret_cast<float4*>(sFlock) + (threadIdx.x >> 5) * kSegments;
     if constexpr (SCAN == 7) {
       float4* cbuf = reinterpret_cast<float4*>(sList + cullBufOffsetWords(ls, A.Mmax)) + (threadIdx.x >> 5) * kCullBufPerWarp;
       n = scanNeighborsCooperative<kCoopCachedRounds, 0, true>(active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd,
-                                                               A.posS, sList, ls, threadIdx.x & ~31u, cbuf);
-    } else if constexpr (SCAN == 8) {
+                                                               A.posS, sList, ls, threadIdx.x & ~31u, segs, cbuf);
+    } else if constexpr (SCAN >= 8) {
       float* dList = reinterpret_cast<float*>(sList + ls * A.Mmax);
-      n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents, false, true>(
-          active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u, nullptr, dList);
+      n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents, false, true, SCAN == 9>(
+          active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u, segs, nullptr, dList);
     } else {
       n = scanNeighborsCooperative<kCoopCachedRounds, SCAN == 5 ? kCoopWindowAgents : 0>(
-          active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u);
+          active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u, segs);
     }
     if (!active) return;
   } else {
@@ -367,6 +371,7 @@ template <int FP, int P2>
 __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];  // (kTileThreads + 1) * Mmax words, a column per thread
   __shared__ float4 sStage[kTileStage];
+  __shared__ float4 sSegs[kTileThreads / 32 * kSegments];
   __shared__ uint32_t sOff[kTileTable], sCnt[kTileTable], sBeg[kTileTable];
   __shared__ uint32_t sScan[kTileThreads / 32 + 1];
   __shared__ uint32_t sTile, sLo, sHi, sStaged;
@@ -466,9 +471,9 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
         const bool inTile = gx >= (int)x0 && gx < (int)(x0 + R) && gy == (int)ty && gz == (int)tz;
         if (active && inTile) n = scanTileStaged(i, p, gx, gy, gz, x0, W, fl, sStage, sOff, sCnt, sList + tid, ls);
       } else {
-        const uint32_t key = fl.cellBase + ((uint32_t)gz * G + (uint32_t)gy) * G + (uint32_t)gx;
-        n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, key, A.flocks, f, A.cellStart,
-                                                                            A.cellEnd, A.posS, sList, ls, tid & ~31u);
+        n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, homeCell(gx, gy, gz, fl), A.flocks,
+                                                                            f, A.cellStart, A.cellEnd, A.posS, sList, ls,
+                                                                            tid & ~31u, sSegs + (tid >> 5) * kSegments);
       }
       if (active) {
         uint32_t* list = sList + tid;
@@ -517,6 +522,7 @@ cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, s
   else if (A.scanVariant == 5) launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 7) launchFlockScan<FP, 7>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 8) launchFlockScan<FP, 8>(A, blocks, block, smem, phase2, regs, st);
+  else if (A.scanVariant == 9) launchFlockScan<FP, 9>(A, blocks, block, smem, phase2, regs, st);
   else launchFlockScan<FP, 0>(A, blocks, block, smem, phase2, regs, st);
   return cudaGetLastError();
 }
@@ -548,6 +554,7 @@ cudaError_t configureFlockFP(int smem, int smemCull, int smemKnn) {
   cudaError_t e = configureCoopScan<FP, 4>(smem);
   if (e == cudaSuccess) e = configureCoopScan<FP, 5>(smem);
   if (e == cudaSuccess) e = configureCoopScan<FP, 8>(smemKnn);
+  if (e == cudaSuccess) e = configureCoopScan<FP, 9>(smemKnn);
   return e == cudaSuccess ? configureCoopScan<FP, 7>(smemCull) : e;
 }
 }  // namespace
@@ -593,13 +600,26 @@ uint32_t tileFlockBlocks(uint32_t Mmax, uint32_t Fs, int smCount) {
   return (uint32_t)(per * std::max(1, smCount));
 }
 
+namespace {
+uint32_t flockSmemWarps(uint32_t block, uint32_t Mmax, int scan) {
+  return (uint32_t)(228u * 1024u / (flockSmemBytes(block, Mmax, scan) + 1024)) * (block / 32u);
+}
+}  // namespace
+// The kNN scan with its run segments in shared memory (8), or in registers (9)
+// where the memory would cost a resident block: 262,144 agents, maxNeighbors 16,
+// 30% in blobs 396 / 409 us a step (three engines), maxNeighbors 30, uniform 288
+// (13 blocks an SM) / 260 (14).
+int flockKnnScan(uint32_t block, uint32_t Mmax, int regs) {
+  const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+  return std::min(byRegs, flockSmemWarps(block, Mmax, 8)) < std::min(byRegs, flockSmemWarps(block, Mmax, 9)) ? 9 : 8;
+}
 // Resident warps: what the register budget allows (flockKernel's launch
 // bounds), or the lists' shared memory.
 uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount) {
   const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
-  const size_t smem = flockSmemBytes(block, A.Mmax, A.scanVariant) + 1024;
-  const uint32_t bySmem = (uint32_t)(228u * 1024u / smem) * (block / 32u);
-  return warpAgentsFor(A.n, smCount * std::min(byRegs, bySmem));
+  const uint32_t resident = std::min(byRegs, flockSmemWarps(block, A.Mmax, A.scanVariant));
+  // Taped steps (the adjoint's forward) run alone: its caller waits for them.
+  return warpAgentsFor(A.n, smCount * resident / (A.taped ? 1u : 2u));
 }
 
 cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs, cudaStream_t st) {

@@ -170,6 +170,7 @@ __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, ui
 template <bool KNN>
 __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
+  __shared__ float4 sSegs[KNN ? 1 : kFusedThreads / 32 * kSegments];
   uint32_t i0;
   const bool active = KNN ? (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n : agentOfLane(A.warpAgents, A.n, i0);
   if (KNN && !active) return;
@@ -185,11 +186,10 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
     n = buildNeighborList<true>(i, xyz(p4), fl, A.cellStart, A.cellEnd, A.posS, list, ls, distL);
   } else {
     const f3 p = xyz(p4);
-    const uint32_t G = fl.G;
-    const uint32_t key = fl.cellBase + ((uint32_t)gridCoord(p.z, fl) * G + (uint32_t)gridCoord(p.y, fl)) * G +
-                         (uint32_t)gridCoord(p.x, fl);
-    n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, key, A.flocks, f, A.cellStart,
-                                                                      A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u);
+    const HomeCell home = homeCell(gridCoord(p.x, fl), gridCoord(p.y, fl), gridCoord(p.z, fl), fl);
+    n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, home, A.flocks, f, A.cellStart,
+                                                                      A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u,
+                                                                      sSegs + (threadIdx.x >> 5) * kSegments);
     if (!active) return;
   }
   const float4 w4 = __ldg(&A.fwdS[i]);
@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
 template <bool KNN>
 __global__ void __launch_bounds__(128) listsKernel(StageArgs A) {
   extern __shared__ uint32_t sList[];
+  __shared__ float4 sSegs[KNN ? 1 : 4 * kSegments];
   uint32_t i0;
   const bool active = KNN ? (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n : agentOfLane(A.warpAgents, A.n, i0);
   if (KNN && !active) return;
@@ -251,12 +252,11 @@ __global__ void __launch_bounds__(128) listsKernel(StageArgs A) {
     float distL[BRT_MAX_NEIGHBORS];
     out[0] = buildNeighborList<true>(i, p, fl, A.cellStart, A.cellEnd, A.posS, out + 1, 1, distL);
   } else {
-    const uint32_t G = fl.G;
-    const uint32_t key = fl.cellBase + ((uint32_t)gridCoord(p.z, fl) * G + (uint32_t)gridCoord(p.y, fl)) * G +
-                         (uint32_t)gridCoord(p.x, fl);
+    const HomeCell home = homeCell(gridCoord(p.x, fl), gridCoord(p.y, fl), gridCoord(p.z, fl), fl);
     const uint32_t ls = blockDim.x + 1;
     const uint32_t n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(
-        active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u);
+        active, i, p, home, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u,
+        sSegs + (threadIdx.x >> 5) * kSegments);
     if (!active) return;
     const uint32_t* list = sList + threadIdx.x;
     for (uint32_t k = 0; k < n; ++k) out[1 + k] = list[k * ls];
@@ -410,7 +410,7 @@ uint32_t residentWarpAgents(const void* fn, int threads, size_t smem, uint32_t n
     cudaGetLastError();
     per = 1;
   }
-  return warpAgentsFor(n, smCount * (uint32_t)(per * threads / 32));
+  return warpAgentsFor(n, smCount * (uint32_t)(per * threads / 32) / 2);
 }
 }  // namespace
 uint32_t fusedWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {

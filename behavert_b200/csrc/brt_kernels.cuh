@@ -63,6 +63,7 @@ struct FusedArgs {
   uint32_t listStride;
   uint32_t nflocks, n, Mmax, Fs;
   uint32_t warpAgents;         // agents a warp of a cooperative scan takes (agentOfLane)
+  bool taped;                  // a step of the adjoint's taped forward or recompute
   float dt;
   int scanVariant;             // 0: pipelined x4 + cell culling, 1: x2 + culling, 2: x4, 3: flat loop,
                                // 4: warp-cooperative, 5: warp-cooperative with windows,
@@ -134,18 +135,21 @@ cudaError_t launchOrderPlace(const OrderArgs& A, cudaStream_t st);
 // warps would leave the GPU part empty.  A warp goes through its home cells'
 // runs one after the other (about 5 us a run of 4 agents), so a launch that
 // does not fill the GPU lasts as long as one warp's chain; 4 agents are about
-// one run.  The line is at one wave of resident warps: with fewer agents a
-// warp the runs are cut into more pieces and the list walk has fewer lanes,
-// which costs more than it saves once every resident slot is taken.  Measured,
-// us a step with 32 / 16 / 8 / 4 agents a warp (maxNeighbors 16, density 1/16,
-// 148 SMs of 32 resident warps): 4,096 agents 59.2 / 48.2 / 42.7 / 39.2;
-// 32,768: 68.0 / 56.6 / 53.2 / 65.5; 65,536: 73.1 / 65.0 / 76.5 / 97.2;
-// 100,003: 83.3 / 90.0 / 100.4 / 131.8.
+// one run.  With fewer agents a warp the runs are cut into more pieces and the
+// list walk has fewer lanes, so the line is at half a wave of resident warps
+// (flockWarpAgents: a full wave where the launch runs alone): a launch alone
+// would gain a little more from a full wave, several engines at once lose by it.
+// Measured, us a step alone with 32 / 16 / 8 / 4 agents a warp (maxNeighbors 16,
+// density 1/16, 148 SMs of 32 resident warps): 4,096 agents 59.2 / 48.2 / 42.7 /
+// 39.2; 16,384: 64.0 / 53.0 / 47.5 / 46.7; 32,768: 68.0 / 56.6 / 53.2 / 65.5;
+// 65,536: 73.1 / 65.0 / 76.5 / 97.2; 100,003: 83.3 / 90.0 / 100.4 / 131.8.  Three
+// engines of 73,029 schooling agents in turn, us a step: 36.5 with 32, 42.0 with 16.
 inline uint32_t warpAgentsFor(uint32_t n, uint32_t residentWarps) {
   for (uint32_t a = 4; a < 32; a *= 2)
     if ((n + a - 1) / a <= residentWarps) return a;
   return 32;
 }
+int flockKnnScan(uint32_t block, uint32_t Mmax, int regs);
 uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount);
 uint32_t fusedWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
 uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);

@@ -153,6 +153,7 @@ __device__ __forceinline__ void copyFeatures(const float* featS, float* featA, u
 // the last agent read-only and leave after the scan.
 __global__ void __launch_bounds__(128) schoolKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
+  __shared__ float4 sSegs[4 * kSegments];
   uint32_t i0;
   const bool active = agentOfLane(A.warpAgents, A.n, i0);
   const uint32_t i = active ? i0 : A.n - 1;
@@ -160,12 +161,11 @@ __global__ void __launch_bounds__(128) schoolKernel(FusedArgs A) {
   const FlockDev& fl = A.flocks[f];
   const float4 p4 = __ldg(&A.posS[i]);
   const f3 p = xyz(p4);
-  const uint32_t G = fl.G;
-  const uint32_t key = fl.cellBase + ((uint32_t)gridCoord(p.z, fl) * G + (uint32_t)gridCoord(p.y, fl)) * G +
-                       (uint32_t)gridCoord(p.x, fl);
+  const HomeCell home = homeCell(gridCoord(p.x, fl), gridCoord(p.y, fl), gridCoord(p.z, fl), fl);
   const uint32_t ls = blockDim.x + 1;  // odd: one vote's rows fall in distinct banks
   const uint32_t n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(
-      active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u);
+      active, i, p, home, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u,
+      sSegs + (threadIdx.x >> 5) * kSegments);
   if (!active) return;
   uint32_t* list = sList + threadIdx.x;
   const float4 w4 = __ldg(&A.fwdS[i]), a4 = __ldg(&A.accS[i]);
@@ -237,7 +237,7 @@ uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
     cudaGetLastError();
     per = 1;
   }
-  return warpAgentsFor(n, smCount * (uint32_t)(per * 4));
+  return warpAgentsFor(n, smCount * (uint32_t)(per * 4) / 2);
 }
 
 cudaError_t launchSchoolStage(const StageArgs& A, int which, cudaStream_t st) {
