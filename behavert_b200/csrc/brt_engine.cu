@@ -825,23 +825,32 @@ int brt_set_state(brt_engine* e, const float* pos4, const float* fwd4, const flo
     BRT_CUDA_TRY(resetOrder(e));
     e->stateLost = false;
   }
-  auto stage4 = [&](const float* src) -> const float4* {
-    if (where == BRT_MEM_DEVICE) return (const float4*)src;
-    cudaMemcpyAsync(e->stage4, src, n * 16, cudaMemcpyHostToDevice, st);
-    return e->stage4;
-  };
   if (n == 0) return BRT_OK;
   // Inputs are in agent-id order; the canonical arrays are in slot order.
-  if (pos4) { const float4* s = stage4(pos4); BRT_CUDA_TRY(launchGatherFromId(s, e->idA, e->posA, e->N, true, st)); }
-  if (fwd4) { const float4* s = stage4(fwd4); BRT_CUDA_TRY(launchGatherFromId(s, e->idA, e->fwdA, e->N, false, st)); }
-  if (acc4) { const float4* s = stage4(acc4); BRT_CUDA_TRY(launchGatherFromId(s, e->idA, e->accA, e->N, false, st)); }
-  if (features && e->Fmax) {
-    const float* s = features;
-    if (where == BRT_MEM_HOST) {
-      BRT_CUDA_TRY(cudaMemcpyAsync(e->stageF, features, n * e->Fmax * 4, cudaMemcpyHostToDevice, st));
-      s = e->stageF;
+  const float* in[3] = {pos4, fwd4, acc4};
+  float4* canon[3] = {e->posA, e->fwdA, e->accA};
+  StateIoArgs S;
+  std::memset(&S, 0, sizeof(S));
+  S.id = e->idA; S.n = e->N; S.F = e->Fmax; S.Fs = e->Fs;
+  if (where == BRT_MEM_DEVICE) {
+    for (int k = 0; k < 3; ++k) { S.src[k] = (const float4*)in[k]; S.dst[k] = canon[k]; }
+    if (features && e->Fmax) { S.featSrc = features; S.featDst = e->featA; }
+    BRT_CUDA_TRY(launchStateIo(S, true, st));
+  } else {
+    // one staging buffer: each array is copied and moved before the next
+    for (int k = 0; k < 3; ++k) {
+      if (!in[k]) continue;
+      BRT_CUDA_TRY(cudaMemcpyAsync(e->stage4, in[k], n * 16, cudaMemcpyHostToDevice, st));
+      S.src[0] = S.src[1] = S.src[2] = nullptr;
+      S.src[k] = e->stage4; S.dst[k] = canon[k];
+      BRT_CUDA_TRY(launchStateIo(S, true, st));
     }
-    BRT_CUDA_TRY(launchGatherFeatFromId(s, e->Fmax, e->idA, e->featA, e->Fs, e->N, st));
+    if (features && e->Fmax) {
+      BRT_CUDA_TRY(cudaMemcpyAsync(e->stageF, features, n * e->Fmax * 4, cudaMemcpyHostToDevice, st));
+      S.src[0] = S.src[1] = S.src[2] = nullptr;
+      S.featSrc = e->stageF; S.featDst = e->featA;
+      BRT_CUDA_TRY(launchStateIo(S, true, st));
+    }
   }
   e->reordered = false;
   e->listsValid = false;
@@ -857,22 +866,29 @@ int brt_get_state(brt_engine* e, float* pos4, float* fwd4, float* acc4, float* f
   cudaStream_t st = e->stream;
   const size_t n = e->N;
   if (n == 0) return BRT_OK;
-  float4* srcs[3] = {e->posA, e->fwdA, e->accA};
-  float* dsts[3] = {pos4, fwd4, acc4};
-  for (int k = 0; k < 3; ++k) {
-    if (!dsts[k]) continue;
-    if (where == BRT_MEM_DEVICE) {
-      BRT_CUDA_TRY(launchScatterToId(srcs[k], e->idA, (float4*)dsts[k], e->N, st));
-    } else {
-      BRT_CUDA_TRY(launchScatterToId(srcs[k], e->idA, e->stage4, e->N, st));
-      BRT_CUDA_TRY(cudaMemcpyAsync(dsts[k], e->stage4, n * 16, cudaMemcpyDeviceToHost, st));
+  const float4* canon[3] = {e->posA, e->fwdA, e->accA};
+  float* out[3] = {pos4, fwd4, acc4};
+  StateIoArgs S;
+  std::memset(&S, 0, sizeof(S));
+  S.id = e->idA; S.n = e->N; S.F = e->Fmax; S.Fs = e->Fs;
+  const bool feats = features && e->Fmax;
+  if (where == BRT_MEM_DEVICE) {
+    for (int k = 0; k < 3; ++k)
+      if (out[k]) { S.src[k] = canon[k]; S.dst[k] = (float4*)out[k]; }
+    if (feats) { S.featSrc = e->featA; S.featDst = features; }
+    BRT_CUDA_TRY(launchStateIo(S, false, st));
+  } else {
+    for (int k = 0; k < 3; ++k) {
+      if (!out[k]) continue;
+      S.src[0] = S.src[1] = S.src[2] = nullptr;
+      S.src[k] = canon[k]; S.dst[k] = e->stage4;
+      BRT_CUDA_TRY(launchStateIo(S, false, st));
+      BRT_CUDA_TRY(cudaMemcpyAsync(out[k], e->stage4, n * 16, cudaMemcpyDeviceToHost, st));
     }
-  }
-  if (features && e->Fmax) {
-    if (where == BRT_MEM_DEVICE) {
-      BRT_CUDA_TRY(launchScatterFeatToId(e->featA, e->Fs, e->idA, features, e->Fmax, e->N, st));
-    } else {
-      BRT_CUDA_TRY(launchScatterFeatToId(e->featA, e->Fs, e->idA, e->stageF, e->Fmax, e->N, st));
+    if (feats) {
+      S.src[0] = S.src[1] = S.src[2] = nullptr;
+      S.featSrc = e->featA; S.featDst = e->stageF;
+      BRT_CUDA_TRY(launchStateIo(S, false, st));
       BRT_CUDA_TRY(cudaMemcpyAsync(features, e->stageF, n * e->Fmax * 4, cudaMemcpyDeviceToHost, st));
     }
   }

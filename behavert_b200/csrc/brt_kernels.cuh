@@ -253,13 +253,18 @@ struct ClusterArgs {
   const float4* in; float4* out;
 };
 cudaError_t launchCluster(const ClusterArgs& A, int which, cudaStream_t st);
-cudaError_t launchScatterToId(const float4* src, const uint32_t* id, float4* dst, uint32_t n, cudaStream_t st);
-cudaError_t launchScatterFeatToId(const float* src, uint32_t Fs, const uint32_t* id, float* dst, uint32_t F, uint32_t n, cudaStream_t st);
-cudaError_t launchLoadFeat(const float* src, uint32_t F, float* dst, uint32_t Fs, uint32_t n, cudaStream_t st);
-cudaError_t launchGatherFromId(const float4* src, const uint32_t* id, float4* dst, uint32_t n, bool forceW1, cudaStream_t st);
+// State between agent-id order and the canonical slot order; a null source
+// leaves its array out.
+struct StateIoArgs {
+  const float4* src[3]; float4* dst[3];  // positions, forwards, smoothed accelerations
+  const float* featSrc; float* featDst;
+  uint32_t F, Fs;                        // floats an agent: outside, and in the canonical array
+  const uint32_t* id;                    // agent id per canonical slot
+  uint32_t n;
+};
+cudaError_t launchStateIo(const StateIoArgs& A, bool gather, cudaStream_t st);
 cudaError_t configureFusedKernels(uint32_t Mmax);
 cudaError_t configureFlockKernels(uint32_t Mmax);
-cudaError_t launchGatherFeatFromId(const float* src, uint32_t F, const uint32_t* id, float* dst, uint32_t Fs, uint32_t n, cudaStream_t st);
 cudaError_t launchHashPairsOut(const uint2* pairs, const uint32_t* idS, uint32_t* keys, uint32_t* ids, uint32_t n, cudaStream_t st);
 // dst[i] = src[index[i * stride]] and dst[index[i]] = src[i] for arrays of
 // `words` 32-bit words per agent.
