@@ -58,6 +58,10 @@ __device__ __forceinline__ f3 separationBar(f3 o, float d2, f3 g) {
   return mul3(sub3(div3(g, d2), mul3(o, 2.0f * dot3(o, g) / (d2 * d2))), -1.0f);
 }
 
+__device__ __forceinline__ f3 shflXor3(uint32_t mask, f3 v, uint32_t o) {
+  return mk3(__shfl_xor_sync(mask, v.x, o), __shfl_xor_sync(mask, v.y, o), __shfl_xor_sync(mask, v.z, o));
+}
+
 // Compensated sum of float3 terms (Knuth's TwoSum per component; exact
 // error terms, since the library is built without contraction).
 struct Comp3 {
@@ -69,6 +73,16 @@ struct Comp3 {
     sum = n;
   }
   __device__ __forceinline__ void add(f3 t) { twoSum(s.x, e.x, t.x); twoSum(s.y, e.y, t.y); twoSum(s.z, e.z, t.z); }
+  // Adds another lane's sum.  Both lanes get the same bits: the sum and its
+  // error are the exact ones either way round, and so is e + o.e.
+  __device__ __forceinline__ void mergeLane(uint32_t mask, uint32_t o) {
+    const f3 os = shflXor3(mask, s, o), oe = shflXor3(mask, e, o);
+    f3 err = mk3(0.f, 0.f, 0.f);
+    twoSum(s.x, err.x, os.x);
+    twoSum(s.y, err.y, os.y);
+    twoSum(s.z, err.z, os.z);
+    e = add3(add3(e, oe), err);
+  }
   __device__ __forceinline__ f3 value() const { return add3(s, e); }
 };
 
@@ -95,8 +109,21 @@ constexpr int kAdjointMinBlocks = 6;
 // Branch bits of the exported flag word (the oracle's frozen-branch layout).
 constexpr uint32_t kBrLow = 1u, kBrLimited = 2u, kBrClipF = 4u, kBrClipV = 8u;
 
+// LANES lanes an agent, lane `sub` taking list entries sub, sub + LANES, ...; what
+// is per agent all its lanes compute alike.  The steering force that decides the
+// branches comes from the tape (the forward's own bits), so nothing here has to
+// follow the list's order but the compensated sums' merge, which is fixed.
+// The kernel waits for its gathers and atomics: more lanes an agent mean shorter
+// chains, and more copies of the per-agent part, so the line is at one wave of
+// resident blocks (launchAdjointStep).  us of emit and gather with 1 / 2 / 4
+// lanes (maxNeighbors 16): 4,096 agents 46 / 34 / 28, 16,384: 49 / 38 / 34,
+// 65,536: 76 / 81 / 81, 64 flocks of 499 k: 433 / 473 / 583; one thread an agent
+// recomputing the forward's sums, 65,536: 77, 499 k: 510.
+template <uint32_t LANES>
 __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointStepKernel(AdjointStepArgs A) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = gt / LANES, sub = gt % LANES;
+  const uint32_t group = ((1u << LANES) - 1u) << (threadIdx.x & 31u & ~(LANES - 1u));  // the agent's lanes
   const bool valid = i < A.n;
   uint32_t f = 0;
   float gw[3] = {0.0f, 0.0f, 0.0f};
@@ -114,22 +141,20 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
     // The adjoint of this step's output.
     const float4 gOp = A.gOutP[i], gOf = A.gOutF[i], gOa = A.gOutA[i];
 
-    // --- forward recomputation (flockingSteer's sequence) -----------------
-    // Two evaluations of the three neighbour sums.  The forward's own order
-    // (x, steer) decides every branch exactly as the forward did.  The
-    // adjoint is linearised at the sums taken in offset form with
-    // compensated (TwoSum) accumulation (xL, steerL): the cohesion sum in
+    // --- the neighbour sums -------------------------------------------------
+    // The forward's steering force (taped) decides every branch exactly as the
+    // forward did.  The adjoint is linearised at the sums taken in offset form
+    // with compensated (TwoSum) accumulation (xL, steerL): the cohesion sum in
     // the forward's form, (sum of positions) / n - own position, cancels
     // coordinates of the world's size down to about one and keeps only
     // ~1e-4 of its value, which the 50-step reverse would amplify.
-    f3 sSep = mk3(0.f, 0.f, 0.f), sAli = mk3(0.f, 0.f, 0.f), sCoh = mk3(0.f, 0.f, 0.f);
     Comp3 cpSep, cpAli, cpCoh;
-    uint32_t cSep = 0, cAli = 0, cCoh = 0, mS = 0, mA = 0, mC = 0;
+    uint32_t mS = 0, mA = 0, mC = 0;
     // Memberships as the flock kernel decides them: with the angle test
     // inactive (cosFree), exact squared-distance thresholds; otherwise the
     // distance and the cosine (both forms decide the same, bit for bit).
     const bool cosFree = dot3(a.fwd, a.fwd) * 1.002f < fl.cosBound2;
-    for (uint32_t k = 0; k < n; ++k) {
+    for (uint32_t k = sub; k < n; k += LANES) {
       const uint32_t j = lst[1 + k];
       const f3 other = neighborImage(a, __ldg(&A.posS[j]), fl);
       const f3 offset = sub3(other, a.pos);
@@ -149,49 +174,42 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
         inC = inBoid(dist, cosAngle, fl.minR, fl.coh[1], fl.coh[2]);
       }
       if (inS) {
-        const f3 t = div3(offset, -d2);
-        sSep = add3(sSep, t);
-        cpSep.add(t);
-        ++cSep;
+        cpSep.add(div3(offset, -d2));
         mS |= 1u << k;
       }
       if (inA) {
-        const f3 fj = xyz(__ldg(&A.fwdS[j]));
-        sAli = add3(sAli, fj);
-        cpAli.add(sub3(fj, a.fwd));
-        ++cAli;
+        cpAli.add(sub3(xyz(__ldg(&A.fwdS[j])), a.fwd));
         mA |= 1u << k;
       }
       if (inC) {
-        sCoh = add3(sCoh, other);
         cpCoh.add(offset);
-        ++cCoh;
         mC |= 1u << k;
       }
     }
+#pragma unroll
+    for (uint32_t o = 1; o < LANES; o <<= 1) {
+      cpSep.mergeLane(group, o);
+      cpAli.mergeLane(group, o);
+      cpCoh.mergeLane(group, o);
+      mS |= __shfl_xor_sync(group, mS, o);
+      mA |= __shfl_xor_sync(group, mA, o);
+      mC |= __shfl_xor_sync(group, mC, o);
+    }
+    const uint32_t cSep = (uint32_t)__popc(mS), cAli = (uint32_t)__popc(mA), cCoh = (uint32_t)__popc(mC);
     const float w[3] = {fl.sep[0], fl.ali[0], fl.coh[0]};
-    f3 x[3], xL[3], u[3], uL[3];
+    const f3 zero = mk3(0.f, 0.f, 0.f);
+    f3 xL[3], uL[3];
     const uint32_t cnt[3] = {cSep, cAli, cCoh};
-    x[0] = cSep ? div3(sSep, (float)cSep) : sSep;
-    x[1] = cAli ? sub3(div3(sAli, (float)cAli), a.fwd) : sAli;
-    x[2] = cCoh ? sub3(div3(sCoh, (float)cCoh), a.pos) : sCoh;
-    xL[0] = cSep ? div3(cpSep.value(), (float)cSep) : sSep;
-    xL[1] = cAli ? div3(cpAli.value(), (float)cAli) : sAli;
-    xL[2] = cCoh ? div3(cpCoh.value(), (float)cCoh) : sCoh;
-    f3 steer = mk3(0.f, 0.f, 0.f), steerL = mk3(0.f, 0.f, 0.f);
+    xL[0] = cSep ? div3(cpSep.value(), (float)cSep) : zero;
+    xL[1] = cAli ? div3(cpAli.value(), (float)cAli) : zero;
+    xL[2] = cCoh ? div3(cpCoh.value(), (float)cCoh) : zero;
+    f3 steer = xyz(__ldg(&A.steerS[i])), steerL = zero;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      u[b] = cnt[b] ? normalize3(x[b]) : x[b];
       uL[b] = cnt[b] ? normalize3(xL[b]) : xL[b];
-      if (w[b] != 0.0f) {
-        steer = add3(mul3(u[b], w[b]), steer);
-        steerL = add3(mul3(uL[b], w[b]), steerL);
-      }
+      if (w[b] != 0.0f) steerL = add3(mul3(uL[b], w[b]), steerL);
     }
-    if (fl.numObstacles && fl.obsW != 0.0f) {
-      steer = obstacleSteer(a, fl, A.obstacles, A.obsMask, steer);
-      steerL = obstacleSteer(a, fl, A.obstacles, A.obsMask, steerL);
-    }
+    if (fl.numObstacles && fl.obsW != 0.0f) steerL = obstacleSteer(a, fl, A.obstacles, A.obsMask, steerL);
 
     f3 gSteer = mk3(0.f, 0.f, 0.f);
     f3 selfP = xyz(gOp), selfF = mk3(0.f, 0.f, 0.f), selfA = xyz(gOa);
@@ -323,7 +341,9 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
     // (a store waiting on its own atomic would otherwise hold up the next
     // entry's atomic).  Positions only place terms the gather sums order-free.
     constexpr int kEmitGroup = 4;
-    for (uint32_t m = mS | mA | mC; m;) {
+    constexpr uint32_t kMine = LANES == 1 ? 0xFFFFFFFFu : (LANES == 2 ? 0x55555555u : 0x11111111u);
+    f3 sent = zero;  // what this lane's entries take from the agent's own position adjoint
+    for (uint32_t m = (mS | mA | mC) & (kMine << sub); m;) {
       uint32_t kk[kEmitGroup], jj[kEmitGroup], q[kEmitGroup];
 #pragma unroll
       for (int u = 0; u < kEmitGroup; ++u) {
@@ -343,7 +363,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
           const f3 o = sub3(other, a.pos);
           const f3 go = separationBar(o, dot3(o, o), gSs);
           gp = add3(gp, go);
-          selfP = sub3(selfP, go);
+          sent = add3(sent, go);
         }
         if ((mC >> k) & 1u) gp = add3(gp, gSc);
         const f3 gf = ((mA >> k) & 1u) ? gSa : mk3(0.f, 0.f, 0.f);
@@ -360,6 +380,10 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
         }
       }
     }
+#pragma unroll
+    for (uint32_t o = 1; o < LANES; o <<= 1) sent = add3(sent, shflXor3(group, sent, o));
+    if (sub != 0) return;
+    selfP = sub3(selfP, sent);
     A.selfP[i] = make_float4(selfP.x, selfP.y, selfP.z, 0.0f);
     A.selfF[i] = make_float4(selfF.x, selfF.y, selfF.z, selfS);
     if (self < A.n) A.gInA[self] = make_float4(selfA.x, selfA.y, selfA.z, 0.0f);
@@ -440,18 +464,21 @@ __device__ __forceinline__ void termsOf(const float4 c0, const float4 c1, float*
   t[0] = c0.x; t[1] = c0.y; t[2] = c0.z; t[3] = c0.w; t[4] = c1.x; t[5] = c1.y;
 }
 
-// kGatherLanes consecutive lanes gather one agent: lane `sub` takes inbox
-// entries sub, sub + kGatherLanes, ... (the group reads the agent's inbox
+// LANES consecutive lanes gather one agent: lane `sub` takes inbox
+// entries sub, sub + LANES, ... (the group reads the agent's inbox
 // block coalesced, once, and keeps its terms in registers for the second
-// pass) and every kGatherLanes-th overflow entry.  The maxima and the
+// pass) and every LANES-th overflow entry.  The maxima and the
 // integer sums combine across the lanes exactly (both are associative), so
 // the split changes no bit.
-constexpr uint32_t kGatherLanes = 8;
-constexpr uint32_t kGatherPerLane = 8;  // inbox entries a lane holds: inCap <= 64
+// Four lanes where they hold the inbox: the scales, the conversions and the
+// combining steps are per lane, and a mean in-list is 17 entries.  us of
+// emit and gather with 8 / 4 lanes: 65,536 agents 84 / 81, 499 k: 524 / 473.
+constexpr uint32_t kGatherPerLane = 8;  // inbox entries a lane holds: inCap <= LANES * 8
 
+template <uint32_t LANES>
 __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGatherKernel(AdjointStepArgs A) {
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t j = gt / kGatherLanes, sub = gt % kGatherLanes;
+  const uint32_t j = gt / LANES, sub = gt % LANES;
   const bool valid = j < A.n;
   uint32_t cnt = 0, head = kNoEntry, inBox = 0;
   float self[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -472,7 +499,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGat
   for (int c = 0; c < 6; ++c) S.mx[c] = fabsf(self[c]);
 #pragma unroll
   for (uint32_t r = 0; r < kGatherPerLane; ++r) {
-    const uint32_t q = sub + r * kGatherLanes;
+    const uint32_t q = sub + r * LANES;
     if (q < inBox) {
       termsOf(box[2 * q], box[2 * q + 1], tk[r]);
       S.seeMax(tk[r]);
@@ -481,27 +508,27 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGat
   float t[6];
   uint32_t r = 0;
   for (uint32_t e = head; e != kNoEntry; e = A.ovNext[e], ++r)
-    if (r % kGatherLanes == sub) { termsOf(A.contrib[2 * (size_t)e], A.contrib[2 * (size_t)e + 1], t); S.seeMax(t); }
+    if (r % LANES == sub) { termsOf(A.contrib[2 * (size_t)e], A.contrib[2 * (size_t)e + 1], t); S.seeMax(t); }
   // the group's maxima (the lanes of one agent are consecutive in the warp)
 #pragma unroll
   for (int c = 0; c < 6; ++c)
 #pragma unroll
-    for (uint32_t o = 1; o < kGatherLanes; o <<= 1) S.mx[c] = fmaxf(S.mx[c], __shfl_xor_sync(0xFFFFFFFFu, S.mx[c], o));
+    for (uint32_t o = 1; o < LANES; o <<= 1) S.mx[c] = fmaxf(S.mx[c], __shfl_xor_sync(0xFFFFFFFFu, S.mx[c], o));
   S.scales(cnt + 1u);
   const bool finite = S.finite;  // the same in every lane of the group (same maxima)
   if (finite) {
     if (sub == 0) S.add(self);
 #pragma unroll
     for (uint32_t rr = 0; rr < kGatherPerLane; ++rr)
-      if (sub + rr * kGatherLanes < inBox) S.add(tk[rr]);
+      if (sub + rr * LANES < inBox) S.add(tk[rr]);
     r = 0;
     for (uint32_t e = head; e != kNoEntry; e = A.ovNext[e], ++r)
-      if (r % kGatherLanes == sub) { termsOf(A.contrib[2 * (size_t)e], A.contrib[2 * (size_t)e + 1], t); S.add(t); }
+      if (r % LANES == sub) { termsOf(A.contrib[2 * (size_t)e], A.contrib[2 * (size_t)e + 1], t); S.add(t); }
   }
 #pragma unroll
   for (int c = 0; c < 6; ++c)
 #pragma unroll
-    for (uint32_t o = 1; o < kGatherLanes; o <<= 1) S.acc[c] += __shfl_xor_sync(0xFFFFFFFFu, S.acc[c], o);
+    for (uint32_t o = 1; o < LANES; o <<= 1) S.acc[c] += __shfl_xor_sync(0xFFFFFFFFu, S.acc[c], o);
   if (!valid || sub != 0) return;
   A.inCount[j] = 0u;  // clean for the next-earlier step
   if (cnt > A.inCap) A.ovHead[j] = kNoEntry;
@@ -632,13 +659,17 @@ __global__ void __launch_bounds__(256) adjointOutKernel(OutArgs A) {
 cudaError_t launchAdjointStep(const AdjointStepArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   if (A.entryStride == 0 || A.entryStride > 32) return cudaErrorInvalidValue;
-  if (A.inCap > kGatherLanes * kGatherPerLane) return cudaErrorInvalidValue;
-  const uint32_t blocks = (A.n + kAdjointThreads - 1) / kAdjointThreads;
-  adjointStepKernel<<<blocks, kAdjointThreads, 0, st>>>(A);
+  if (A.inCap > 8 * kGatherPerLane || !A.steerS) return cudaErrorInvalidValue;
+  const auto blocksOf = [&](uint32_t lanes) { return (uint32_t)(((size_t)A.n * lanes + kAdjointThreads - 1) / kAdjointThreads); };
+  // the most lanes whose blocks are resident at once (148 SMs of kAdjointMinBlocks)
+  constexpr uint32_t kWave = 148u * kAdjointMinBlocks;
+  if (blocksOf(4) <= kWave) adjointStepKernel<4><<<blocksOf(4), kAdjointThreads, 0, st>>>(A);
+  else if (blocksOf(2) <= kWave) adjointStepKernel<2><<<blocksOf(2), kAdjointThreads, 0, st>>>(A);
+  else adjointStepKernel<1><<<blocksOf(1), kAdjointThreads, 0, st>>>(A);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  const uint32_t gatherBlocks = (uint32_t)(((size_t)A.n * kGatherLanes + kAdjointThreads - 1) / kAdjointThreads);
-  adjointGatherKernel<<<gatherBlocks, kAdjointThreads, 0, st>>>(A);
+  if (A.inCap <= 4 * kGatherPerLane) adjointGatherKernel<4><<<blocksOf(4), kAdjointThreads, 0, st>>>(A);
+  else adjointGatherKernel<8><<<blocksOf(8), kAdjointThreads, 0, st>>>(A);
   return cudaGetLastError();
 }
 cudaError_t launchFlockReduce(const FlockReduceArgs& A, cudaStream_t st) {

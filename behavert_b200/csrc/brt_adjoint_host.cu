@@ -41,7 +41,8 @@ struct AdjointState {
   // two k-step tapes: the backward recomputes segment c - 1 into one while
   // the reverse of segment c reads the other
   struct Tape {
-    float4 *pos = nullptr, *fwd = nullptr, *acc = nullptr;
+    char* mem = nullptr;  // the allocation that the arrays are carved from
+    float4 *pos = nullptr, *fwd = nullptr, *acc = nullptr, *steer = nullptr;
     uint32_t *prev = nullptr, *id = nullptr, *lists = nullptr;
   } tape[2];
   // the reverse chain's stream and the events that order it against the
@@ -118,7 +119,7 @@ int checkSupported(brt_engine* e) {
 bool wholeTapeFits(brt_engine* e, uint32_t T) {
   if (e->adjointCheckpoints) return false;
   if (T <= e->adj->capK[0]) return true;  // there already
-  const size_t step = (size_t)e->N * (3 * 16 + 2 * 4 + 4 * (size_t)e->listStride);
+  const size_t step = (size_t)e->N * (4 * 16 + 2 * 4 + 4 * (size_t)e->listStride);
   size_t freeBytes = 0, total = 0;
   if (cudaMemGetInfo(&freeBytes, &total) != cudaSuccess) {
     cudaGetLastError();
@@ -183,11 +184,17 @@ int ensureCapacity(brt_engine* e, uint32_t nck, uint32_t k, uint32_t T, bool who
     AdjointState::Tape& t = a->tape[i];
     a->capK[i] = 0;
     changed = true;
-    if ((rc = regrow(&t.pos, n * k)) || (rc = regrow(&t.fwd, n * k)) || (rc = regrow(&t.acc, n * k)) ||
-        (rc = regrow(&t.prev, n * k)) || (rc = regrow(&t.id, n * k)) || (rc = regrow(&t.lists, n * k * e->listStride))) {
+    // one allocation: seven of this size would take several times as long
+    const size_t parts[7] = {n * k * 16, n * k * 16, n * k * 16, n * k * 16, n * k * 4, n * k * 4, n * k * e->listStride * 4};
+    size_t at[8] = {0};
+    for (int p = 0; p < 7; ++p) at[p + 1] = at[p] + ((parts[p] + 255) & ~(size_t)255);
+    if ((rc = regrow(&t.mem, at[7]))) {
       dropGraphs(a);
       return rc;
     }
+    t.pos = (float4*)(t.mem + at[0]); t.fwd = (float4*)(t.mem + at[1]); t.acc = (float4*)(t.mem + at[2]);
+    t.steer = (float4*)(t.mem + at[3]);
+    t.prev = (uint32_t*)(t.mem + at[4]); t.id = (uint32_t*)(t.mem + at[5]); t.lists = (uint32_t*)(t.mem + at[6]);
     a->capK[i] = k;
   }
   if (!a->revStream) BRT_CUDA_TRY(cudaStreamCreateWithFlags(&a->revStream, cudaStreamNonBlocking));
@@ -236,10 +243,12 @@ int enqueueTaped(brt_engine* e, uint32_t steps, const AdjointState::Tape& tp, bo
     e->idS = tp.id + s * n;
     e->lists = tp.lists + s * n * e->listStride;
     e->tapePrev = tp.prev + s * n;
+    e->tapeSteer = tp.steer + s * n;
     rc = engineEnqueueStep(e, a->dt, true);
   }
   e->posS = posS; e->fwdS = fwdS; e->accS = accS; e->idS = idS; e->lists = lists;
   e->tapePrev = nullptr;
+  e->tapeSteer = nullptr;
   e->userFrozen = wasFrozen;
   return rc;
 }
@@ -327,6 +336,7 @@ int enqueueBackward(brt_engine* e, uint32_t variant) {
       AdjointStepArgs R;
       std::memset(&R, 0, sizeof(R));
       R.posS = tp.pos + s * n; R.fwdS = tp.fwd + s * n; R.accS = tp.acc + s * n;
+      R.steerS = tp.steer + s * n;
       R.lists = tp.lists + s * n * e->listStride; R.listStride = e->listStride;
       R.prev = tp.prev + s * n; R.idS = tp.id + s * n;
       R.flocks = e->flocks; R.agentBase = e->agentBase; R.obstacles = e->obstacles; R.obsMask = e->obsMask;

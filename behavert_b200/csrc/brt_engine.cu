@@ -356,7 +356,7 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   bool twoPass = e->forceTwoPass || (e->anyKnn && e->Mmax > 32);
   for (const FlockDev& d : e->flocksHost) twoPass = twoPass || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
   if (e->anyKnn && !twoPass) F.scanVariant = flockKnnScan(e->fusedBlock, e->Mmax, e->regBudget);
-  F.taped = e->tapePrev != nullptr;
+  F.steerOut = e->tapeSteer;
   F.warpAgents = e->school ? e->schoolWarp
                  : twoPass ? e->fusedWarp
                            : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);

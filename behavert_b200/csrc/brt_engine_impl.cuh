@@ -89,6 +89,7 @@ struct brt_engine {
   uint64_t timedSteps = 0;
   // adjoint (brt_adjoint_host.cu): tape slot of the reorder's source slots
   uint32_t* tapePrev = nullptr;
+  float4* tapeSteer = nullptr;  // and of the flock kernel's steering forces
   brt::AdjointState* adj = nullptr;
   bool adjointGraphs = true;  // option "adjoint_graphs"
   bool adjointExport = false; // option "adjoint_export"

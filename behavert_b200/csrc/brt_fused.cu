@@ -203,6 +203,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
     steer = add3(mul3(sCoh, fl.coh[0]), steer);
   }
   if (fl.numObstacles && fl.obsW != 0.0f) steer = obstacleSteer(a, fl, A.obstacles, A.obsMask, steer);
+  if (A.steerOut) A.steerOut[i] = make_float4(steer.x, steer.y, steer.z, 0.0f);
   if (FP > 0) {
     if (relaxOn && n > 0 && sumS > 0.0f) {
 #pragma unroll
@@ -619,7 +620,7 @@ uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t 
   const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
   const uint32_t resident = std::min(byRegs, flockSmemWarps(block, A.Mmax, A.scanVariant));
   // Taped steps (the adjoint's forward) run alone: its caller waits for them.
-  return warpAgentsFor(A.n, smCount * resident / (A.taped ? 1u : 2u));
+  return warpAgentsFor(A.n, smCount * resident / (A.steerOut ? 1u : 2u));
 }
 
 cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs, cudaStream_t st) {

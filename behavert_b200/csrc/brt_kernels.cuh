@@ -55,6 +55,7 @@ struct FusedArgs {
   const float* featS; const uint32_t* idS;
   float4* posA; float4* fwdA; float4* accA; float* featA; uint32_t* idA;
   float4* statsById;
+  float4* steerOut;            // optional: the steering force of every sorted slot (adjoint tape)
   const uint32_t* cellStart; const uint32_t* cellEnd;
   const FlockDev* flocks; const uint32_t* agentBase;
   const float4* obstacles;
@@ -63,7 +64,6 @@ struct FusedArgs {
   uint32_t listStride;
   uint32_t nflocks, n, Mmax, Fs;
   uint32_t warpAgents;         // agents a warp of a cooperative scan takes (agentOfLane)
-  bool taped;                  // a step of the adjoint's taped forward or recompute
   float dt;
   int scanVariant;             // 0: pipelined x4 + cell culling, 1: x2 + culling, 2: x4, 3: flat loop,
                                // 4: warp-cooperative, 5: warp-cooperative with windows,
@@ -160,6 +160,7 @@ uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
 constexpr uint32_t kAdjointThreads = 128;
 struct AdjointStepArgs {
   const float4* posS; const float4* fwdS; const float4* accS;   // the step's sorted input state
+  const float4* steerS;                                          // and the steering force of its forward
   const uint32_t* lists; uint32_t listStride;                    // its neighbour lists (sorted slots)
   const uint32_t* prev;                                          // canonical slot of each sorted slot
   const uint32_t* idS;                                           // agent id per sorted slot
