@@ -121,6 +121,7 @@ constexpr uint32_t kBrLow = 1u, kBrLimited = 2u, kBrClipF = 4u, kBrClipV = 8u;
 // recomputing the forward's sums, 65,536: 77, 499 k: 510.
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointStepKernel(AdjointStepArgs A) {
+  chainBegin();
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t i = gt / LANES, sub = gt % LANES;
   const uint32_t group = ((1u << LANES) - 1u) << (threadIdx.x & 31u & ~(LANES - 1u));  // the agent's lanes
@@ -477,6 +478,7 @@ constexpr uint32_t kGatherPerLane = 8;  // inbox entries a lane holds: inCap <= 
 
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGatherKernel(AdjointStepArgs A) {
+  chainBegin();
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t j = gt / LANES, sub = gt % LANES;
   const bool valid = j < A.n;
@@ -663,14 +665,13 @@ cudaError_t launchAdjointStep(const AdjointStepArgs& A, cudaStream_t st) {
   const auto blocksOf = [&](uint32_t lanes) { return (uint32_t)(((size_t)A.n * lanes + kAdjointThreads - 1) / kAdjointThreads); };
   // the most lanes whose blocks are resident at once (148 SMs of kAdjointMinBlocks)
   constexpr uint32_t kWave = 148u * kAdjointMinBlocks;
-  if (blocksOf(4) <= kWave) adjointStepKernel<4><<<blocksOf(4), kAdjointThreads, 0, st>>>(A);
-  else if (blocksOf(2) <= kWave) adjointStepKernel<2><<<blocksOf(2), kAdjointThreads, 0, st>>>(A);
-  else adjointStepKernel<1><<<blocksOf(1), kAdjointThreads, 0, st>>>(A);
-  cudaError_t err = cudaGetLastError();
+  cudaError_t err;
+  if (blocksOf(4) <= kWave) err = launchChained(A.n, adjointStepKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
+  else if (blocksOf(2) <= kWave) err = launchChained(A.n, adjointStepKernel<2>, blocksOf(2), kAdjointThreads, 0, st, A);
+  else err = launchChained(A.n, adjointStepKernel<1>, blocksOf(1), kAdjointThreads, 0, st, A);
   if (err != cudaSuccess) return err;
-  if (A.inCap <= 4 * kGatherPerLane) adjointGatherKernel<4><<<blocksOf(4), kAdjointThreads, 0, st>>>(A);
-  else adjointGatherKernel<8><<<blocksOf(8), kAdjointThreads, 0, st>>>(A);
-  return cudaGetLastError();
+  if (A.inCap <= 4 * kGatherPerLane) return launchChained(A.n, adjointGatherKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
+  return launchChained(A.n, adjointGatherKernel<8>, blocksOf(8), kAdjointThreads, 0, st, A);
 }
 cudaError_t launchFlockReduce(const FlockReduceArgs& A, cudaStream_t st) {
   if (A.nflocks == 0) return cudaSuccess;

@@ -228,6 +228,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
 template <int FP, int P2, int MINB, int SCAN>
 __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs A) {
   extern __shared__ __align__(16) uint32_t sFlock[];
+  chainBegin();
   uint32_t* sList = sFlock + (SCAN >= 4 && SCAN != 9 ? (blockDim.x >> 5) * kSegments * 4u : 0u);
   // The warp-cooperative scans need every lane of the warp; inactive lanes
   // take part read-only (mirroring the last agent) and leave after it.
@@ -493,39 +494,36 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
 
 namespace {
 template <int FP, int SCAN>
-void launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
+cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
                      cudaStream_t st) {
   if constexpr (SCAN == 0) {
     if (phase2 == 1) {
-      if (regs > 64) flockKernel<FP, 1, 2, 0><<<blocks, block, smem, st>>>(A);
-      else flockKernel<FP, 1, 4, 0><<<blocks, block, smem, st>>>(A);
-      return;
+      if (regs > 64) return launchChained(A.n, flockKernel<FP, 1, 2, 0>, blocks, block, smem, st, A);
+      else return launchChained(A.n, flockKernel<FP, 1, 4, 0>, blocks, block, smem, st, A);
     }
   }
   if constexpr (SCAN >= 4 && FP > 0) {
     if (phase2 == 2) {
-      if (regs <= 48) flockKernel<FP, 2, 5, SCAN><<<blocks, block, smem, st>>>(A);
-      else flockKernel<FP, 2, 4, SCAN><<<blocks, block, smem, st>>>(A);
-      return;
+      if (regs <= 48) return launchChained(A.n, flockKernel<FP, 2, 5, SCAN>, blocks, block, smem, st, A);
+      else return launchChained(A.n, flockKernel<FP, 2, 4, SCAN>, blocks, block, smem, st, A);
     }
   }
   if constexpr (SCAN >= 4) {
-    if (regs <= 40) { flockKernel<FP, 0, 6, SCAN><<<blocks, block, smem, st>>>(A); return; }
-    if (regs <= 48) { flockKernel<FP, 0, 5, SCAN><<<blocks, block, smem, st>>>(A); return; }
+    if (regs <= 40) return launchChained(A.n, flockKernel<FP, 0, 6, SCAN>, blocks, block, smem, st, A);
+    if (regs <= 48) return launchChained(A.n, flockKernel<FP, 0, 5, SCAN>, blocks, block, smem, st, A);
   }
-  if (regs > 64) flockKernel<FP, 0, 2, SCAN><<<blocks, block, smem, st>>>(A);
-  else flockKernel<FP, 0, 4, SCAN><<<blocks, block, smem, st>>>(A);
+  if (regs > 64) return launchChained(A.n, flockKernel<FP, 0, 2, SCAN>, blocks, block, smem, st, A);
+  else return launchChained(A.n, flockKernel<FP, 0, 4, SCAN>, blocks, block, smem, st, A);
 }
 template <int FP>
 cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
                           cudaStream_t st) {
-  if (A.scanVariant == 4) launchFlockScan<FP, 4>(A, blocks, block, smem, phase2, regs, st);
-  else if (A.scanVariant == 5) launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
-  else if (A.scanVariant == 7) launchFlockScan<FP, 7>(A, blocks, block, smem, phase2, regs, st);
-  else if (A.scanVariant == 8) launchFlockScan<FP, 8>(A, blocks, block, smem, phase2, regs, st);
-  else if (A.scanVariant == 9) launchFlockScan<FP, 9>(A, blocks, block, smem, phase2, regs, st);
-  else launchFlockScan<FP, 0>(A, blocks, block, smem, phase2, regs, st);
-  return cudaGetLastError();
+  if (A.scanVariant == 4) return launchFlockScan<FP, 4>(A, blocks, block, smem, phase2, regs, st);
+  else if (A.scanVariant == 5) return launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
+  else if (A.scanVariant == 7) return launchFlockScan<FP, 7>(A, blocks, block, smem, phase2, regs, st);
+  else if (A.scanVariant == 8) return launchFlockScan<FP, 8>(A, blocks, block, smem, phase2, regs, st);
+  else if (A.scanVariant == 9) return launchFlockScan<FP, 9>(A, blocks, block, smem, phase2, regs, st);
+  return launchFlockScan<FP, 0>(A, blocks, block, smem, phase2, regs, st);
 }
 template <int FP, int SCAN>
 cudaError_t configureCoopScan(int smem) {

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) hashKernel(HashArgs A) {
 // members of a cell of more than kRankLimit are in id order already).
 template <bool RANK>
 __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
+  chainBegin();
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gstride = gridDim.x * blockDim.x;
   if (!RANK)
@@ -171,6 +172,7 @@ template <bool KNN>
 __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
   __shared__ float4 sSegs[KNN ? 1 : kFusedThreads / 32 * kSegments];
+  chainBegin();
   uint32_t i0;
   const bool active = KNN ? (i0 = blockIdx.x * blockDim.x + threadIdx.x) < A.n : agentOfLane(A.warpAgents, A.n, i0);
   if (KNN && !active) return;
@@ -399,12 +401,10 @@ cudaError_t launchHash(const HashArgs& A, uint32_t smBlocks, cudaStream_t st) {
 }
 cudaError_t launchReorder(const ReorderArgs& A, cudaStream_t st) {
   if (A.members) {
-    reorderKernel<true><<<std::max(1u, blocksFor(A.n, 256)), 256, 0, st>>>(A);
-  } else {
-    const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
-    reorderKernel<false><<<blocks, 256, 0, st>>>(A);
+    return launchChained(A.n, reorderKernel<true>, std::max(1u, blocksFor(A.n, 256)), 256, 0, st, A);
   }
-  return cudaGetLastError();
+  const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
+  return launchChained(A.n, reorderKernel<false>, blocks, 256, 0, st, A);
 }
 cudaError_t configureFusedKernels(uint32_t Mmax) {
   const int smem = (int)((size_t)(kFusedThreads + 1) * Mmax * 4);
@@ -433,9 +433,8 @@ uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
 cudaError_t launchFused(const FusedArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const size_t smem = (size_t)(kFusedThreads + 1) * A.Mmax * 4;
-  if (knn) fusedKernel<true><<<blocksFor(A.n, kFusedThreads), kFusedThreads, smem, st>>>(A);
-  else fusedKernel<false><<<blocksFor(A.n, kFusedThreads / 32 * A.warpAgents), kFusedThreads, smem, st>>>(A);
-  return cudaGetLastError();
+  if (knn) return launchChained(A.n, fusedKernel<true>, blocksFor(A.n, kFusedThreads), kFusedThreads, smem, st, A);
+  return launchChained(A.n, fusedKernel<false>, blocksFor(A.n, kFusedThreads / 32 * A.warpAgents), kFusedThreads, smem, st, A);
 }
 cudaError_t launchLists(const StageArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;

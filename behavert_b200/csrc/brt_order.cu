@@ -79,6 +79,7 @@ __device__ __forceinline__ uint32_t ctaExclusiveScan(uint32_t v, uint32_t* sWarp
 // a cell: one atomic a run of equal cells (its first lane adds the run's
 // length), about a quarter of one an agent at 4 agents a cell.
 __global__ void __launch_bounds__(256) countKernel(OrderArgs A, uint32_t cellTiles) {
+  chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < cellTiles) A.tileStatus[j] = 0u;
   if (j == 0) {
@@ -111,6 +112,7 @@ template <uint32_t THREADS, uint32_t ITEMS>
 __global__ void __launch_bounds__(THREADS) cellScanKernel(OrderArgs A) {
   __shared__ uint32_t sTile, sPrefix;
   __shared__ uint32_t sWarp[THREADS / 32 + 1];
+  chainBegin();
   if (threadIdx.x == 0) sTile = atomicAdd(&A.words[kOrderWordTile], 1u);
   __syncthreads();
   const uint32_t tile = sTile;
@@ -263,6 +265,7 @@ __device__ void sortBigCell(const OrderArgs& A, uint32_t s, uint32_t e, uint32_t
 
 __global__ void __launch_bounds__(kPlaceThreads) placeKernel(OrderArgs A, uint32_t blocks) {
   __shared__ bool sLast;
+  chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t big = A.words[kOrderWordBig];
   if (j < A.n) {
@@ -304,22 +307,22 @@ uint32_t orderCellTiles(uint32_t numCells) {
 cudaError_t launchOrderCount(const OrderArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const uint32_t tiles = orderCellTiles(A.numCells);
-  countKernel<<<(std::max(A.n, tiles) + 255) / 256, 256, 0, st>>>(A, tiles);
-  return cudaGetLastError();
+  return launchChained(A.n, countKernel, (std::max(A.n, tiles) + 255) / 256, 256, 0, st, A, tiles);
 }
 
 cudaError_t launchOrderPlace(const OrderArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const uint32_t tiles = orderCellTiles(A.numCells);
+  cudaError_t e;
   switch (cellScanTile(A.numCells)) {
-    case 256: cellScanKernel<256, 1><<<tiles, 256, 0, st>>>(A); break;
-    case 512: cellScanKernel<256, 2><<<tiles, 256, 0, st>>>(A); break;
-    case 1024: cellScanKernel<256, 4><<<tiles, 256, 0, st>>>(A); break;
-    default: cellScanKernel<1024, 8><<<tiles, 1024, 0, st>>>(A); break;
+    case 256: e = launchChained(A.n, cellScanKernel<256, 1>, tiles, 256, 0, st, A); break;
+    case 512: e = launchChained(A.n, cellScanKernel<256, 2>, tiles, 256, 0, st, A); break;
+    case 1024: e = launchChained(A.n, cellScanKernel<256, 4>, tiles, 256, 0, st, A); break;
+    default: e = launchChained(A.n, cellScanKernel<1024, 8>, tiles, 1024, 0, st, A); break;
   }
+  if (e != cudaSuccess) return e;
   const uint32_t blocks = (A.n + kPlaceThreads - 1) / kPlaceThreads;
-  placeKernel<<<blocks, kPlaceThreads, 0, st>>>(A, blocks);
-  return cudaGetLastError();
+  return launchChained(A.n, placeKernel, blocks, kPlaceThreads, 0, st, A, blocks);
 }
 
 }  // namespace brt

@@ -154,6 +154,7 @@ __device__ __forceinline__ void copyFeatures(const float* featS, float* featA, u
 __global__ void __launch_bounds__(128) schoolKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
   __shared__ float4 sSegs[4 * kSegments];
+  chainBegin();
   uint32_t i0;
   const bool active = agentOfLane(A.warpAgents, A.n, i0);
   const uint32_t i = active ? i0 : A.n - 1;
@@ -227,8 +228,7 @@ __global__ void __launch_bounds__(128) schoolStageKernel(StageArgs A, int which)
 cudaError_t launchSchool(const FusedArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const uint32_t block = 128, blockAgents = block / 32 * A.warpAgents;
-  schoolKernel<<<(A.n + blockAgents - 1) / blockAgents, block, (size_t)(block + 1) * A.Mmax * 4, st>>>(A);
-  return cudaGetLastError();
+  return launchChained(A.n, schoolKernel, (A.n + blockAgents - 1) / blockAgents, block, (size_t)(block + 1) * A.Mmax * 4, st, A);
 }
 
 uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
