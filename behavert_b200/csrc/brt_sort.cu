@@ -31,6 +31,7 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kFlagMask = 3u << 30;
 constexpr uint32_t kValMask = (1u << 30) - 1;
+constexpr int kAhead = 8;  // predecessors a look-back reads at once
 
 // Exclusive scan of one value per thread across the CTA; returns the
 // exclusive prefix and writes the total to *total.
@@ -76,7 +77,7 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
   constexpr int TILE = (int)sortTileFor(BITS);
   constexpr int DPT = (BINS + T - 1) / T;  // digits per thread (consecutive)
 
-  __shared__ uint32_t sWarp[WARPS][BINS];
+  __shared__ uint16_t sWarp[WARPS][BINS];
   __shared__ uint32_t sDigitStart[BINS];
   __shared__ uint32_t sGlobal[BINS];
   __shared__ uint2 sItems[TILE];
@@ -85,7 +86,7 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) sTile = atomicAdd(counter, 1u);
-  for (int k = tid; k < WARPS * BINS; k += T) (&sWarp[0][0])[k] = 0u;
+  for (int k = tid; k < WARPS * BINS; k += T) (&sWarp[0][0])[k] = 0;
   __syncthreads();
   const uint32_t tile = sTile;
   const uint32_t tileBase = tile * (uint32_t)TILE;
@@ -117,7 +118,7 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
     uint32_t base = 0;
     if (lane == leader && d < (uint32_t)BINS) {
       base = sWarp[warp][d];
-      sWarp[warp][d] = base + __popc(peers);
+      sWarp[warp][d] = (uint16_t)(base + __popc(peers));
     }
     base = __shfl_sync(0xffffffffu, base, leader);
     off[i] = base + __popc(peers & ltmask);
@@ -135,7 +136,7 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) {
         uint32_t t = sWarp[w][d];
-        sWarp[w][d] = run;
+        sWarp[w][d] = (uint16_t)run;
         run += t;
       }
       // Publish as early as possible so successors can proceed.
@@ -167,21 +168,30 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
         int p = (int)tile - 1;
         uint32_t spins = 0;
         const bool stalled = tile == wait.stallTile;
-        while (p >= 0) {
-          const uint32_t v = stalled ? 0u : ldRelaxed(&status[(size_t)p * BINS + d]);
-          const uint32_t f = v & kFlagMask;
-          if (f == 0u) {
-            // Plain bounded polling: a predecessor that has claimed its tile
-            // is resident and publishes within microseconds.
-            if (++spins > wait.spinLimit) {
-              atomicOr(errWord, kDevErrLookback);
-              break;
-            }
-            continue;
+        // kAhead predecessors' words are asked for at once: tiles that start
+        // together find up to dozens of partial counts before a full prefix,
+        // and one dependent load after the other took most of a pass
+        for (bool done = false; !done;) {
+          uint32_t v[kAhead];
+#pragma unroll
+          for (int q = 0; q < kAhead; ++q)  // before tile 0 there is nothing: a full prefix of zero
+            v[q] = p >= q ? (stalled ? 0u : ldRelaxed(&status[(size_t)(p - q) * BINS + d])) : kFlagInc;
+          int used = 0;
+#pragma unroll
+          for (int q = 0; q < kAhead; ++q) {
+            const uint32_t f = v[q] & kFlagMask;
+            if (done || used < q || f == 0u) continue;  // used < q: an earlier one is not published yet
+            excl += v[q] & kValMask;
+            done = f == kFlagInc;
+            ++used;
           }
-          excl += v & kValMask;
-          if (f == kFlagInc) break;
-          --p;
+          p -= used;
+          // Plain bounded polling: a predecessor that has claimed its tile is
+          // resident and publishes within microseconds.
+          if (!done && used < kAhead && ++spins > wait.spinLimit) {
+            atomicOr(errWord, kDevErrLookback);
+            break;
+          }
         }
         stRelaxed(&status[(size_t)tile * BINS + d], kFlagInc | ((excl + cnt[k]) & kValMask));
       }
@@ -212,19 +222,42 @@ onesweepKernel(const uint2* __restrict__ in, uint2* __restrict__ out, uint32_t n
   }
 }
 
+// Digit counts of every pass; also clears the error word.  `wide`: the input is
+// 16-byte aligned, and a thread takes two pairs a load, four loads at a time.
 template <int BITS>
 __global__ void __launch_bounds__(256)
 histogramKernel(const uint2* __restrict__ in, uint32_t n, uint32_t passes, uint32_t digitBits,
-                uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3, uint32_t* __restrict__ hist) {
+                uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3, uint32_t* __restrict__ hist, uint32_t* errWord, bool wide) {
   constexpr int BINS = 1 << BITS;
   __shared__ uint32_t sh[4 * BINS];
   for (int k = threadIdx.x; k < 4 * BINS; k += blockDim.x) sh[k] = 0u;
+  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  if (gtid == 0) *errWord = 0u;
   __syncthreads();
   const uint32_t masks[4] = {m0, m1, m2, m3};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t key = in[i].x;
+  auto count = [&](uint32_t key) {
     for (uint32_t p = 0; p < passes; ++p) atomicAdd(&sh[p * BINS + ((key >> (p * digitBits)) & masks[p])], 1u);
+  };
+  uint32_t first = 0;
+  if (wide) {
+    const uint4* in2 = reinterpret_cast<const uint4*>(in);
+    const uint32_t n2 = n / 2;
+    uint32_t i = gtid;
+    for (; i < n2 && n2 - i > 3 * stride; i += 4 * stride) {
+      uint4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = __ldg(&in2[i + q * stride]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { count(v[q].x); count(v[q].z); }
+    }
+    for (; i < n2; i += stride) {
+      const uint4 v = __ldg(&in2[i]);
+      count(v.x);
+      count(v.z);
+    }
+    first = n2 * 2;
   }
+  for (uint32_t i = first + gtid; i < n; i += stride) count(in[i].x);
   __syncthreads();
   for (uint32_t k = threadIdx.x; k < passes * BINS; k += blockDim.x)
     if (sh[k]) atomicAdd(&hist[k], sh[k]);
@@ -296,13 +329,14 @@ cudaError_t launchOnesweepPass(const SortPlan& p, uint32_t pass, const uint2* in
   return cudaGetLastError();
 }
 
-cudaError_t launchSortHistogram(const SortPlan& p, const uint2* in, const SortScratch& s, cudaStream_t st) {
+cudaError_t launchSortHistogram(const SortPlan& p, const uint2* in, const SortScratch& s, uint32_t* errWord, cudaStream_t st) {
   if (p.n == 0) return cudaSuccess;
   uint32_t m[4] = {0, 0, 0, 0};
   for (uint32_t k = 0; k < p.passes; ++k) m[k] = passMask(p, k);
-  uint32_t blocks = std::min<uint32_t>((p.n + 255) / 256, 148u * 8u);
+  const bool wide = ((uintptr_t)in & 15u) == 0;
+  uint32_t blocks = std::min<uint32_t>((p.n + (wide ? 511u : 255u)) / (wide ? 512u : 256u), 148u * 4u);
   switch (p.digitBits) {
-#define BRT_HIST_CASE(B) case B: histogramKernel<B><<<blocks, 256, 0, st>>>(in, p.n, p.passes, p.digitBits, m[0], m[1], m[2], m[3], s.hist); break;
+#define BRT_HIST_CASE(B) case B: histogramKernel<B><<<blocks, 256, 0, st>>>(in, p.n, p.passes, p.digitBits, m[0], m[1], m[2], m[3], s.hist, errWord, wide); break;
     BRT_HIST_CASE(4) BRT_HIST_CASE(5) BRT_HIST_CASE(6) BRT_HIST_CASE(7) BRT_HIST_CASE(8) BRT_HIST_CASE(9)
 #undef BRT_HIST_CASE
     default: return cudaErrorInvalidValue;
@@ -335,9 +369,9 @@ extern "C" int brt_radix_sort_pairs(const uint32_t* pairs_in, uint32_t* pairs_ou
   cudaStream_t st = (cudaStream_t)stream;
   brt::SortScratch s = brt::carveSortScratch(p, scratch, true);
   uint32_t* err = (uint32_t*)((char*)scratch + s.bytes);
-  BRT_CUDA_TRY(cudaMemsetAsync(scratch, 0, s.bytes - (size_t)n * 8 + 4, st));
-  BRT_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
-  BRT_CUDA_TRY(brt::launchSortHistogram(p, (const uint2*)pairs_in, s, st));
+  // histogram, tile counters and look-back words; the histogram kernel clears the error word
+  BRT_CUDA_TRY(cudaMemsetAsync(scratch, 0, (size_t)((char*)s.tmp - (char*)scratch), st));
+  BRT_CUDA_TRY(brt::launchSortHistogram(p, (const uint2*)pairs_in, s, err, st));
   // Ping-pong so that the last pass writes pairs_out.
   const uint2* src = (const uint2*)pairs_in;
   for (uint32_t k = 0; k < p.passes; ++k) {
@@ -427,11 +461,10 @@ extern "C" int brt_radix_sort_pairs_noalloc(const uint32_t* pairs_in, uint32_t* 
   brt::SortScratch s = brt::carveSortScratch(p, base, true);
   uint32_t* err = (uint32_t*)((char*)base + s.bytes);
   // The array keeps the previous call's contents: clear the histogram, tile
-  // counters, look-back status and error word (the ping-pong half is fully
-  // overwritten before it is read).
+  // counters and look-back status (the histogram kernel clears the error word,
+  // the ping-pong half is fully overwritten before it is read).
   BRT_CUDA_TRY(cudaMemsetAsync(base, 0, (size_t)((char*)s.tmp - (char*)base), st));
-  BRT_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
-  BRT_CUDA_TRY(brt::launchSortHistogram(p, (const uint2*)pairs_in, s, st));
+  BRT_CUDA_TRY(brt::launchSortHistogram(p, (const uint2*)pairs_in, s, err, st));
   const uint2* src = (const uint2*)pairs_in;
   for (uint32_t k = 0; k < p.passes; ++k) {
     uint2* dst = (((p.passes - 1 - k) & 1u) == 0u) ? (uint2*)pairs_out : s.tmp;
