@@ -350,11 +350,12 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   F.tiles = e->tiles; F.numTiles = e->numTiles; F.tileCounter = e->tileCounter; F.tileBlocks = e->tileBlocks;
   F.stepCounter = e->stepCounter;
   F.cullGate = (e->scanVariant == 0 || e->scanVariant == 1) ? e->cullWords + 2 : nullptr;
-  // The single-pass kernel covers every flock unless one needs clustering
-  // steering (it needs the whole list first) or kNN lists longer than a warp.
-  // kNN flocks take its cooperative kNN scan (scan 8).
-  bool twoPass = e->forceTwoPass || (e->anyKnn && e->Mmax > 32);
-  for (const FlockDev& d : e->flocksHost) twoPass = twoPass || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
+  // The single-pass kernel covers every flock unless one needs kNN lists longer
+  // than a warp, or some need kNN and some clustering steering.  kNN flocks
+  // take its cooperative kNN scan (scan 8 or 9), clustering ones its scan 5.
+  for (const FlockDev& d : e->flocksHost) F.clus = F.clus || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
+  const bool twoPass = e->forceTwoPass || (e->anyKnn && (e->Mmax > 32 || F.clus));
+  if (!twoPass && F.clus) F.scanVariant = 5;
   if (e->anyKnn && !twoPass) F.scanVariant = flockKnnScan(e->fusedBlock, e->Mmax, e->regBudget);
   F.steerOut = e->tapeSteer;
   F.warpAgents = e->school ? e->schoolWarp

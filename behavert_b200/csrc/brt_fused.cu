@@ -1,5 +1,6 @@
-// brt_fused.cu -- the fused flocking kernel for flocks without kNN
-// replacement or clustering steering (those use fusedKernel, brt_kernels.cu).
+// brt_fused.cu -- the fused flocking kernel: flocking, kNN lists of at most a
+// warp, clustering steering (kNN and clustering flocks in one engine, and longer
+// kNN lists, use fusedKernel, brt_kernels.cu).
 //
 // One thread per sorted slot.  Phase 1 scans the 27 neighbour cells in the
 // reference's visit order (Proximity3D_kernel.cu:108-115) into a shared-memory
@@ -53,7 +54,14 @@ __host__ __device__ constexpr size_t flockSmemBytes(uint32_t block, uint32_t Mma
 // then the clustering feature update and the integration of sorted slot i
 // into canonical slot i.  Shared by flockKernel and tileFlockKernel, so
 // every scan variant walks and integrates with the same code.
-template <int FP, int P2>
+//
+// CLUS: flocks with clustering steering (clusteringSteer: BehaviorClustering
+// split path, BehaviorClustering_kernel.cu:306-497).  Its similarity is the
+// feature pass's, its running statistics go through the list in order, and its
+// two sums are independent of the others', so all of it belongs in that one
+// pass: each neighbour's features are read once instead of twice, its norm comes
+// with its position, and no similarity is stored.
+template <int FP, int P2, bool CLUS = false>
 __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const float4 p4, const FlockDev& fl,
                                           const uint32_t* list, uint32_t ls, uint32_t n) {
   const f3 p = xyz(p4);
@@ -118,8 +126,17 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
       ++cCoh;
     }
   };
-  auto visitFeat = [&](const float* fj, float n2) {
-    if (relaxOn) {
+  const bool clusCoh = CLUS && F > 0 && fl.clus != 0.0f, clusAli = CLUS && F > 0 && fl.aclus != 0.0f;
+  const bool clusOn = clusCoh || clusAli;
+  f3 sClus = mk3(0.f, 0.f, 0.f), sClusAli = mk3(0.f, 0.f, 0.f);
+  float4 stats = make_float4(0.f, 0.f, 0.f, 0.f);
+  uint32_t id = 0;
+  if (CLUS && clusOn) {
+    id = __ldg(&A.idS[i]);
+    stats = A.statsById[id];
+  }
+  auto visitFeat = [&](const float* fj, float n2, uint32_t j, const float4 q4) {
+    if (relaxOn || clusOn) {
       // computeSimilarity's dot product, then acc += s * f_j, in the
       // reference's sequential order.  Scalar on purpose: ptxas -O3 for
       // sm_100a contracts a packed FP32 multiply feeding a packed add into a
@@ -129,17 +146,31 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
 #pragma unroll
       for (int kk = 0; kk < FP; ++kk) dot += fi[kk] * fj[kk];
       const float s = (dot / (n1 * n2) + 1.0f) / 2.0f;
-      sumS += s;
+      if (!CLUS || relaxOn) {
+        sumS += s;
 #pragma unroll
-      for (int kk = 0; kk < FP; ++kk) facc[kk] += s * fj[kk];
+        for (int kk = 0; kk < FP; ++kk) facc[kk] += s * fj[kk];
+      }
+      if (CLUS && clusOn) {
+        stats = updateSimilarityStats(s, stats, fl);
+        const float sim = interpolateSimilarity(s, stats.x, stats.y, stats.z);
+        if (clusCoh) {
+          // seek and flee: the offset and its exact negative, cut to the same length
+          const f3 to = truncateLength(sub3(neighborImage(a, q4, fl), p), fl.maxSpeed);
+          const f3 myVel = mul3(fwd, w4.w);
+          const f3 seek = sub3(to, myVel), flee = sub3(mk3(-to.x, -to.y, -to.z), myVel);
+          sClus = add3(sClus, add3(mul3(seek, sim), mul3(flee, 1.0f - sim)));
+        }
+        if (clusAli) sClusAli = add3(sClusAli, mul3(xyz(__ldg(&A.fwdS[j])), sim));
+      }
     }
   };
   auto visit = [&](const float4 q4, const float4 wj, const float* fj, float n2) {
     visitGeom(q4, wj);
-    visitFeat(fj, n2);
+    visitFeat(fj, n2, 0u, q4);
   };
   auto loadFeat = [&](uint32_t j, float* fj) {
-    if (relaxOn) {
+    if (relaxOn || clusOn) {
       const float4* src = reinterpret_cast<const float4*>(A.featS) + (size_t)j * fs4;
 #pragma unroll
       for (int qq = 0; qq < FP / 4; ++qq) {
@@ -166,12 +197,13 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
       const uint32_t j = list[k * ls];
       visitGeom(__ldg(&A.posS[j]), aliOn ? __ldg(&A.fwdS[j]) : zero4);
     }
-    if (relaxOn) {
+    if (relaxOn || clusOn) {
       for (uint32_t k = 0; k < n; ++k) {
         const uint32_t j = list[k * ls];
         float fj[FP > 0 ? FP : 1];
         loadFeat(j, fj);
-        visitFeat(fj, __ldg(&A.posS[j]).w);
+        const float4 q = __ldg(&A.posS[j]);
+        visitFeat(fj, q.w, j, q);
       }
     }
   } else {
@@ -202,6 +234,17 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
     if (cCoh > 0) sCoh = normalize3(sub3(div3(sCoh, (float)cCoh), p));
     steer = add3(mul3(sCoh, fl.coh[0]), steer);
   }
+  if (CLUS && clusOn) {
+    A.statsById[id] = stats;
+    if (clusCoh) {
+      if (n > 0) sClus = mul3(normalize3(div3(sClus, (float)n)), fl.clus);
+      steer = add3(sClus, steer);
+    }
+    if (clusAli) {
+      if (n > 0) sClusAli = mul3(normalize3(sub3(div3(sClusAli, (float)n), fwd)), fl.aclus);
+      steer = add3(sClusAli, steer);
+    }
+  }
   if (fl.numObstacles && fl.obsW != 0.0f) steer = obstacleSteer(a, fl, A.obstacles, A.obsMask, steer);
   if (A.steerOut) A.steerOut[i] = make_float4(steer.x, steer.y, steer.z, 0.0f);
   if (FP > 0) {
@@ -225,7 +268,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
   A.idA[i] = __ldg(&A.idS[i]);
 }
 
-template <int FP, int P2, int MINB, int SCAN>
+template <int FP, int P2, int MINB, int SCAN, bool CLUS = false>
 __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs A) {
   extern __shared__ __align__(16) uint32_t sFlock[];
   chainBegin();
@@ -286,7 +329,7 @@ __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs 
     for (uint32_t k = 0; k < n; ++k) out[1 + k] = list[k * ls];
   }
 
-  flockWalk<FP, P2>(A, i, p4, fl, list, ls, n);
+  flockWalk<FP, P2, CLUS>(A, i, p4, fl, list, ls, n);
 }
 
 // Exclusive scan of one value per thread across a kTileThreads block.
@@ -492,6 +535,10 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
   }
 }
 
+// Resident 256-thread blocks an SM the clustering instantiations are compiled for
+// (80 registers).  131,072 agents, 8 features, us a step: 142 alone, 85 with three
+// engines in turn; the list-first kernel 185 and 141, with 32 features 316 / 775.
+constexpr int kClusBlocks = 3;
 namespace {
 template <int FP, int SCAN>
 cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
@@ -518,6 +565,9 @@ cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block,
 template <int FP>
 cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
                           cudaStream_t st) {
+  if constexpr (FP > 0) {
+    if (A.clus) return launchChained(A.n, flockKernel<FP, 2, kClusBlocks, 5, true>, blocks, block, smem, st, A);
+  }
   if (A.scanVariant == 4) return launchFlockScan<FP, 4>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 5) return launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 7) return launchFlockScan<FP, 7>(A, blocks, block, smem, phase2, regs, st);
@@ -552,6 +602,10 @@ cudaError_t configureFlockFP(int smem, int smemCull, int smemKnn) {
   }
   cudaError_t e = configureCoopScan<FP, 4>(smem);
   if (e == cudaSuccess) e = configureCoopScan<FP, 5>(smem);
+  if constexpr (FP > 0) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(flockKernel<FP, 2, kClusBlocks, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  }
   if (e == cudaSuccess) e = configureCoopScan<FP, 8>(smemKnn);
   if (e == cudaSuccess) e = configureCoopScan<FP, 9>(smemKnn);
   return e == cudaSuccess ? configureCoopScan<FP, 7>(smemCull) : e;
@@ -615,7 +669,7 @@ int flockKnnScan(uint32_t block, uint32_t Mmax, int regs) {
 // Resident warps: what the register budget allows (flockKernel's launch
 // bounds), or the lists' shared memory.
 uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount) {
-  const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+  const uint32_t byRegs = A.clus ? 8u * kClusBlocks : regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
   const uint32_t resident = std::min(byRegs, flockSmemWarps(block, A.Mmax, A.scanVariant));
   // Taped steps (the adjoint's forward) run alone: its caller waits for them.
   return warpAgentsFor(A.n, smCount * resident / (A.steerOut ? 1u : 2u));

@@ -162,8 +162,9 @@ __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, ui
   for (uint32_t k = 0; k < F; ++k) fi[k] = __ldg(&src[k]);
 }
 
-// Fused neighbour search + flocking steering + clustering + obstacles +
-// feature relaxation + integration.  Lists stay in shared memory
+// The list-first kernel (option "two_pass", kNN lists above a warp, kNN and
+// clustering flocks in one engine): neighbour search, flocking steering,
+// clustering, obstacles, feature relaxation, integration.  Lists stay in shared memory
 // ([k][thread] layout, odd stride) unless recording is on.  First-M lists
 // come from the warp-cooperative windowed scan (every lane of a warp takes
 // part; inactive lanes mirror the last agent read-only and leave after it),

@@ -55,6 +55,7 @@ struct FusedArgs {
   const float* featS; const uint32_t* idS;
   float4* posA; float4* fwdA; float4* accA; float* featA; uint32_t* idA;
   float4* statsById;
+  bool clus;                   // some flock has clustering steering
   float4* steerOut;            // optional: the steering force of every sorted slot (adjoint tape)
   const uint32_t* cellStart; const uint32_t* cellEnd;
   const FlockDev* flocks; const uint32_t* agentBase;
