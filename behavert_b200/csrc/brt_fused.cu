@@ -535,10 +535,21 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
   }
 }
 
-// Resident 256-thread blocks an SM the clustering instantiations are compiled for
-// (80 registers).  131,072 agents, 8 features, us a step: 142 alone, 85 with three
-// engines in turn; the list-first kernel 185 and 141, with 32 features 316 / 775.
-constexpr int kClusBlocks = 3;
+// Resident 256-thread blocks an SM the clustering instantiations are compiled for:
+// 2 (128 registers, next to no spills) for more than 8 features, and where all
+// warps are resident at once even so; else 3 (80 registers).  us a step alone
+// with 2 / 3 / 4: 8 features 4,096 agents 41 / 44 / 47, 65,536: 77 / 81 / 96,
+// 400,000: 366 / 302 / 316; 32 features 4,096: 55 / 78 / 86, 400,000: 580 / 734 / 745.
+// The list-first kernel: 8 features 97, 138, 521; 32 features 206, 2445.
+inline uint32_t clusBlocks(uint32_t features4, uint32_t n) {
+  return features4 > 8u || n <= 148u * 16u * 32u ? 2u : 3u;
+}
+// Resident 256-thread blocks an SM of walk 2 at the default register budget: with
+// more features, fewer blocks and fewer spills.  us a step with 4 / 3 / 2 blocks:
+// 12 features (16 in registers) 4,096 agents 54 / 47 / 45, 262,144: 273 / 250 / 285,
+// 1,048,576: 856 / 796 / 968; 32 features 4,096: 87 / 65 / 53, 1,048,576: 1887 /
+// 1619 / 1338.
+constexpr int walk2Blocks(int FP) { return FP > 16 ? 2 : (FP > 8 ? 3 : 4); }
 namespace {
 template <int FP, int SCAN>
 cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
@@ -552,7 +563,7 @@ cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block,
   if constexpr (SCAN >= 4 && FP > 0) {
     if (phase2 == 2) {
       if (regs <= 48) return launchChained(A.n, flockKernel<FP, 2, 5, SCAN>, blocks, block, smem, st, A);
-      else return launchChained(A.n, flockKernel<FP, 2, 4, SCAN>, blocks, block, smem, st, A);
+      else return launchChained(A.n, flockKernel<FP, 2, walk2Blocks(FP), SCAN>, blocks, block, smem, st, A);
     }
   }
   if constexpr (SCAN >= 4) {
@@ -566,7 +577,11 @@ template <int FP>
 cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
                           cudaStream_t st) {
   if constexpr (FP > 0) {
-    if (A.clus) return launchChained(A.n, flockKernel<FP, 2, kClusBlocks, 5, true>, blocks, block, smem, st, A);
+    if constexpr (FP <= 8) {
+      if (A.clus && clusBlocks(A.Fs, A.n) == 3u)
+        return launchChained(A.n, flockKernel<FP, 2, 3, 5, true>, blocks, block, smem, st, A);
+    }
+    if (A.clus) return launchChained(A.n, flockKernel<FP, 2, 2, 5, true>, blocks, block, smem, st, A);
   }
   if (A.scanVariant == 4) return launchFlockScan<FP, 4>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 5) return launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
@@ -584,7 +599,7 @@ cudaError_t configureCoopScan(int smem) {
     if (e != cudaSuccess) return e;
   }
   if constexpr (FP > 0) {
-    const void* split[2] = {(const void*)flockKernel<FP, 2, 4, SCAN>, (const void*)flockKernel<FP, 2, 5, SCAN>};
+    const void* split[2] = {(const void*)flockKernel<FP, 2, walk2Blocks(FP), SCAN>, (const void*)flockKernel<FP, 2, 5, SCAN>};
     for (const void* fn : split) {
       cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (e != cudaSuccess) return e;
@@ -604,7 +619,11 @@ cudaError_t configureFlockFP(int smem, int smemCull, int smemKnn) {
   if (e == cudaSuccess) e = configureCoopScan<FP, 5>(smem);
   if constexpr (FP > 0) {
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(flockKernel<FP, 2, kClusBlocks, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      e = cudaFuncSetAttribute(flockKernel<FP, 2, 2, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if constexpr (FP <= 8) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(flockKernel<FP, 2, 3, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    }
   }
   if (e == cudaSuccess) e = configureCoopScan<FP, 8>(smemKnn);
   if (e == cudaSuccess) e = configureCoopScan<FP, 9>(smemKnn);
@@ -669,7 +688,8 @@ int flockKnnScan(uint32_t block, uint32_t Mmax, int regs) {
 // Resident warps: what the register budget allows (flockKernel's launch
 // bounds), or the lists' shared memory.
 uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount) {
-  const uint32_t byRegs = A.clus ? 8u * kClusBlocks : regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+  const uint32_t byRegs = A.clus ? 8u * clusBlocks(A.Fs, A.n)
+                          : regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
   const uint32_t resident = std::min(byRegs, flockSmemWarps(block, A.Mmax, A.scanVariant));
   // Taped steps (the adjoint's forward) run alone: its caller waits for them.
   return warpAgentsFor(A.n, smCount * resident / (A.steerOut ? 1u : 2u));
