@@ -121,6 +121,7 @@ constexpr uint32_t kBrLow = 1u, kBrLimited = 2u, kBrClipF = 4u, kBrClipV = 8u;
 // recomputing the forward's sums, 65,536: 77, 499 k: 510.
 template <uint32_t LANES>
 __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointStepKernel(AdjointStepArgs A) {
+  constexpr bool CHAIN = LANES == 4;  // the other instantiations are never launched chained
   chainBegin();
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t i = gt / LANES, sub = gt % LANES;
@@ -131,13 +132,13 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
   if (valid) {
     f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
     const FlockDev& fl = A.flocks[f];
-    const float4 p4 = __ldg(&A.posS[i]);
-    const float4 w4 = __ldg(&A.fwdS[i]);
-    const float4 a4 = __ldg(&A.accS[i]);
+    const float4 p4 = ldStep<CHAIN>(&A.posS[i]);
+    const float4 w4 = ldStep<CHAIN>(&A.fwdS[i]);
+    const float4 a4 = ldStep<CHAIN>(&A.accS[i]);
     const AgentCtx a = makeCtx(p4, w4, fl);
     const uint32_t* lst = A.lists + (size_t)i * A.listStride;
     const uint32_t n = lst[0];
-    const uint32_t self = __ldg(&A.prev[i]);
+    const uint32_t self = ldStep<CHAIN>(&A.prev[i]);
 
     // The adjoint of this step's output.
     const float4 gOp = A.gOutP[i], gOf = A.gOutF[i], gOa = A.gOutA[i];
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
     const bool cosFree = dot3(a.fwd, a.fwd) * 1.002f < fl.cosBound2;
     for (uint32_t k = sub; k < n; k += LANES) {
       const uint32_t j = lst[1 + k];
-      const f3 other = neighborImage(a, __ldg(&A.posS[j]), fl);
+      const f3 other = neighborImage(a, ldStep<CHAIN>(&A.posS[j]), fl);
       const f3 offset = sub3(other, a.pos);
       const float d2 = dot3(offset, offset);
       bool inS, inA, inC;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
         mS |= 1u << k;
       }
       if (inA) {
-        cpAli.add(sub3(xyz(__ldg(&A.fwdS[j])), a.fwd));
+        cpAli.add(sub3(xyz(ldStep<CHAIN>(&A.fwdS[j])), a.fwd));
         mA |= 1u << k;
       }
       if (inC) {
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
     xL[0] = cSep ? div3(cpSep.value(), (float)cSep) : zero;
     xL[1] = cAli ? div3(cpAli.value(), (float)cAli) : zero;
     xL[2] = cCoh ? div3(cpCoh.value(), (float)cCoh) : zero;
-    f3 steer = xyz(__ldg(&A.steerS[i])), steerL = zero;
+    f3 steer = xyz(ldStep<CHAIN>(&A.steerS[i])), steerL = zero;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       uL[b] = cnt[b] ? normalize3(xL[b]) : xL[b];
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
         const uint32_t k = kk[u], j = jj[u];
         f3 gp = mk3(0.f, 0.f, 0.f);
         if ((mS >> k) & 1u) {
-          const f3 other = neighborImage(a, __ldg(&A.posS[j]), fl);
+          const f3 other = neighborImage(a, ldStep<CHAIN>(&A.posS[j]), fl);
           const f3 o = sub3(other, a.pos);
           const f3 go = separationBar(o, dot3(o, o), gSs);
           gp = add3(gp, go);
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
     A.selfF[i] = make_float4(selfF.x, selfF.y, selfF.z, selfS);
     if (self < A.n) A.gInA[self] = make_float4(selfA.x, selfA.y, selfA.z, 0.0f);
 
-    const uint32_t id = __ldg(&A.idS[i]);
+    const uint32_t id = ldStep<CHAIN>(&A.idS[i]);
     double* acc = A.accW + 3 * (size_t)id;
     acc[0] += (double)gw[0];
     acc[1] += (double)gw[1];
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointSte
       reinterpret_cast<uint4*>(A.exportFlags)[id] = make_uint4(br, mS, mA, mC);
       uint32_t* row = A.exportLists + (size_t)id * A.listStride;
       row[0] = n;
-      for (uint32_t k = 0; k < n; ++k) row[1 + k] = __ldg(&A.idS[lst[1 + k]]);
+      for (uint32_t k = 0; k < n; ++k) row[1 + k] = ldStep<CHAIN>(&A.idS[lst[1 + k]]);
     }
     if (A.exportState) {
       A.exportState[3 * (size_t)id + 0] = p4;
@@ -485,7 +486,9 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGat
   uint32_t cnt = 0, head = kNoEntry, inBox = 0;
   float self[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   float selfS = 0.0f;
+  uint32_t tj = 0;
   if (valid) {
+    tj = ldStep<true>(&A.prev[j]);
     cnt = A.inCount[j];
     inBox = min(cnt, A.inCap);
     if (cnt > A.inCap) head = A.ovHead[j];
@@ -553,7 +556,6 @@ __global__ void __launch_bounds__(kAdjointThreads, kAdjointMinBlocks) adjointGat
       for (int c = 0; c < 6; ++c) res[c] += t[c];
     }
   }
-  const uint32_t tj = __ldg(&A.prev[j]);
   if (tj >= A.n) return;  // only a corrupted step leaves such a source slot
   A.gInP[tj] = make_float4(res[0], res[1], res[2], 0.0f);
   A.gInF[tj] = make_float4(res[3], res[4], res[5], selfS);
@@ -667,8 +669,8 @@ cudaError_t launchAdjointStep(const AdjointStepArgs& A, cudaStream_t st) {
   constexpr uint32_t kWave = 148u * kAdjointMinBlocks;
   cudaError_t err;
   if (blocksOf(4) <= kWave) err = launchChained(A.n, adjointStepKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
-  else if (blocksOf(2) <= kWave) err = launchChained(A.n, adjointStepKernel<2>, blocksOf(2), kAdjointThreads, 0, st, A);
-  else err = launchChained(A.n, adjointStepKernel<1>, blocksOf(1), kAdjointThreads, 0, st, A);
+  else if (blocksOf(2) <= kWave) err = launchPlain(adjointStepKernel<2>, blocksOf(2), kAdjointThreads, 0, st, A);
+  else err = launchPlain(adjointStepKernel<1>, blocksOf(1), kAdjointThreads, 0, st, A);
   if (err != cudaSuccess) return err;
   if (A.inCap <= 4 * kGatherPerLane) return launchChained(A.n, adjointGatherKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
   return launchChained(A.n, adjointGatherKernel<8>, blocksOf(8), kAdjointThreads, 0, st, A);

@@ -17,7 +17,7 @@ namespace brt {
 // d2 <= r2thr (sqrtf is monotone and correctly rounded, r2thr is the largest
 // float whose root does not exceed the radius).  With kNN off the scan stops
 // once M entries are held: later candidates cannot change the list.
-template <bool KNN>
+template <bool CHAIN, bool KNN>
 __device__ __forceinline__ uint32_t buildNeighborList(uint32_t self, f3 p, const FlockDev& fl,
                                                       const uint32_t* __restrict__ cellStart,
                                                       const uint32_t* __restrict__ cellEnd,
@@ -39,13 +39,13 @@ __device__ __forceinline__ uint32_t buildNeighborList(uint32_t self, f3 p, const
         const int cz = wrapCoord(gz + oz, fl.G);
         const float sz = imageShift(gz, oz, fl.G, fl.L);
         const uint32_t h = fl.cellBase + ((uint32_t)cz * fl.G + (uint32_t)cy) * fl.G + (uint32_t)cx;
-        const uint32_t start = __ldg(&cellStart[h]);
-        uint32_t stop = __ldg(&cellEnd[h]);
+        const uint32_t start = ldStep<CHAIN>(&cellStart[h]);
+        uint32_t stop = ldStep<CHAIN>(&cellEnd[h]);
         if (!usableRange(fl, start, stop)) continue;
         if (fl.maxPerCell && stop - start > fl.maxPerCell) stop = start + fl.maxPerCell;
         for (uint32_t j = start; j < stop; ++j) {
           if (j == self) continue;
-          const float4 q = __ldg(&posS[j]);
+          const float4 q = ldStep<CHAIN>(&posS[j]);
           const float dx = (q.x + sx) - p.x, dy = (q.y + sy) - p.y, dz = (q.z + sz) - p.z;
           const float d2 = dx * dx + dy * dy + dz * dz;
           if (!knn) {
@@ -346,7 +346,7 @@ __device__ __forceinline__ HomeCell homeCell(int gx, int gy, int gz, const Flock
   return {fl.cellBase + ((uint32_t)gz * fl.G + (uint32_t)gy) * fl.G + (uint32_t)gx,
           (uint32_t)gx | (uint32_t)gy << 10 | (uint32_t)gz << 20};
 }
-template <int R, int WINT = 0, bool CULL = false, bool KNN = false, bool SEGREG = false>
+template <bool CHAIN, int R, int WINT = 0, bool CULL = false, bool KNN = false, bool SEGREG = false>
 __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32_t self, f3 p, HomeCell home,
                                                              const FlockDev* __restrict__ flocks, uint32_t flock,
                                                              const uint32_t* __restrict__ cellStart,
@@ -421,7 +421,7 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
     if (lane < 27u) {
       const int cx = wrapCoord(gx + ox, G), cy = wrapCoord(gy + oy, G), cz = wrapCoord(gz + oz, G);
       const uint32_t h = cellBase + ((uint32_t)cz * G + (uint32_t)cy) * G + (uint32_t)cx;
-      const uint32_t st = __ldg(&cellStart[h]), en = __ldg(&cellEnd[h]);
+      const uint32_t st = ldStep<CHAIN>(&cellStart[h]), en = ldStep<CHAIN>(&cellEnd[h]);
       if (st < en && st >= slotLo && en <= slotHi) {  // usableRange
         segStart = st;
         segLen = min(en - st, most);
@@ -486,7 +486,7 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
               const float4 seg = segmentOf(base0 + (uint32_t)r * 32u);
               if (t < total) {
                 cslot[r] = __float_as_uint(seg.x) + t;
-                const float4 q = __ldg(&posS[cslot[r]]);
+                const float4 q = ldStep<CHAIN>(&posS[cslot[r]]);
                 cqx[r] = q.x + seg.y;
                 cqy[r] = q.y + seg.z;
                 cqz[r] = q.z + seg.w;
@@ -613,7 +613,7 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
           float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
           if (t < total) {
             const uint32_t slot = __float_as_uint(seg.x) + t;
-            const float4 q = __ldg(&posS[slot]);
+            const float4 q = ldStep<CHAIN>(&posS[slot]);
             v = make_float4(q.x + seg.y, q.y + seg.z, q.z + seg.w, __uint_as_float(slot));
             const float ex = fmaxf(fmaxf(lx - v.x, v.x - hx), 0.0f);
             const float ey = fmaxf(fmaxf(ly - v.y, v.y - hy), 0.0f);
@@ -696,7 +696,7 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
             const float4 seg = segmentOf(base0 + (uint32_t)r * 32u);
             if (t < total) {
               cslot[r] = __float_as_uint(seg.x) + t;
-              const float4 q = __ldg(&posS[cslot[r]]);
+              const float4 q = ldStep<CHAIN>(&posS[cslot[r]]);
               cqx[r] = q.x + seg.y;
               cqy[r] = q.y + seg.z;
               cqz[r] = q.z + seg.w;
@@ -736,7 +736,7 @@ __device__ __forceinline__ uint32_t scanNeighborsCooperative(bool active, uint32
       const bool valid = t < total;
       const float4 seg = segmentOf(base);
       const uint32_t slot = valid ? __float_as_uint(seg.x) + t : 0xFFFFFFFFu;
-      const float4 q = valid ? __ldg(&posS[slot]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 q = valid ? ldStep<CHAIN>(&posS[slot]) : make_float4(0.f, 0.f, 0.f, 0.f);
       const float qx = q.x + seg.y, qy = q.y + seg.z, qz = q.z + seg.w;
       for (uint32_t todo = open; todo; todo &= todo - 1u) {
         const uint32_t a = __ffs(todo) - 1u;
@@ -816,6 +816,7 @@ __device__ __forceinline__ bool inBoid(float dist, float cosAngle, float minR, f
 // (calcSeparation :166-211, calcAlignment :253-290, calcCohesion :216-249),
 // and the results are blended in the flocking demo's order
 // (BehaveRT_Flocking.cpp:183-193): steer = ((0 + sep*w) + ali*w) + coh*w.
+template <bool CHAIN>
 __device__ __forceinline__ f3 flockingSteer(const AgentCtx& a, const FlockDev& fl, const uint32_t* list, uint32_t ls,
                                             uint32_t n, const float4* __restrict__ posS, const float4* __restrict__ fwdS,
                                             f3 steer, bool SEP, bool ALI, bool COH) {
@@ -823,7 +824,7 @@ __device__ __forceinline__ f3 flockingSteer(const AgentCtx& a, const FlockDev& f
   uint32_t cSep = 0, cAli = 0, cCoh = 0;
   for (uint32_t k = 0; k < n; ++k) {
     const uint32_t j = list[k * ls];
-    const f3 other = neighborImage(a, __ldg(&posS[j]), fl);
+    const f3 other = neighborImage(a, ldStep<CHAIN>(&posS[j]), fl);
     const f3 offset = sub3(other, a.pos);
     const float d2 = dot3(offset, offset);
     const float dist = sqrtf(d2);
@@ -834,7 +835,7 @@ __device__ __forceinline__ f3 flockingSteer(const AgentCtx& a, const FlockDev& f
       ++cSep;
     }
     if (ALI && inBoid(dist, cosAngle, fl.minR, fl.ali[1], fl.ali[2])) {
-      sAli = add3(sAli, xyz(__ldg(&fwdS[j])));
+      sAli = add3(sAli, xyz(ldStep<CHAIN>(&fwdS[j])));
       ++cAli;
     }
     if (COH && inBoid(dist, cosAngle, fl.minR, fl.coh[1], fl.coh[2])) {
@@ -900,10 +901,11 @@ __device__ __forceinline__ f3 avoidNeighbors(const AgentCtx& a, const FlockDev& 
 
 // computeSimilarity (BehaviorClustering_resources.cu:156-180); the self norm
 // is the same for every pair and is passed in.
+template <bool CHAIN>
 __device__ __forceinline__ float similarity(const float* fi, float norm1, const float* __restrict__ fj, uint32_t F) {
   float dot = 0.0f, n2 = 0.0f;
   for (uint32_t k = 0; k < F; ++k) {
-    const float b = __ldg(&fj[k]);
+    const float b = ldStep<CHAIN>(&fj[k]);
     dot += fi[k] * b;
     n2 += b * b;
   }
@@ -958,13 +960,14 @@ __device__ __forceinline__ f3 truncateLength(f3 v, float maxLength) {
 // BehaviorClustering_resources.cu:269-384): adaptive similarity per
 // neighbour, then cluster cohesion (seek/flee blend) and cluster alignment,
 // each blended into the steering force.  Similarities are staged in `sims`.
+template <bool CHAIN>
 __device__ __forceinline__ f3 clusteringSteer(const AgentCtx& a, const FlockDev& fl, const uint32_t* list, uint32_t ls, uint32_t n,
                                               const float4* __restrict__ posS, const float4* __restrict__ fwdS,
                                               const float* fi, float norm1, const float* __restrict__ featS,
                                               uint32_t Fs, float4& stats, float* sims, f3 steer) {
   const bool coh = fl.clus != 0.0f, ali = fl.aclus != 0.0f;
   for (uint32_t k = 0; k < n; ++k) {
-    const float s = similarity(fi, norm1, featS + (size_t)list[k * ls] * Fs, fl.F);
+    const float s = similarity<CHAIN>(fi, norm1, featS + (size_t)list[k * ls] * Fs, fl.F);
     stats = updateSimilarityStats(s, stats, fl);
     sims[k] = interpolateSimilarity(s, stats.x, stats.y, stats.z);
   }
@@ -973,7 +976,7 @@ __device__ __forceinline__ f3 clusteringSteer(const AgentCtx& a, const FlockDev&
     const f3 myVel = mul3(a.fwd, a.speed);
     for (uint32_t k = 0; k < n; ++k) {
       const float sim = sims[k];
-      const f3 other = neighborImage(a, __ldg(&posS[list[k * ls]]), fl);
+      const f3 other = neighborImage(a, ldStep<CHAIN>(&posS[list[k * ls]]), fl);
       const f3 seek = sub3(truncateLength(sub3(other, a.pos), fl.maxSpeed), myVel);
       const f3 flee = sub3(truncateLength(sub3(a.pos, other), fl.maxSpeed), myVel);
       const float om = 1.0f - sim;
@@ -984,7 +987,7 @@ __device__ __forceinline__ f3 clusteringSteer(const AgentCtx& a, const FlockDev&
   }
   if (ali) {
     f3 s = mk3(0.f, 0.f, 0.f);
-    for (uint32_t k = 0; k < n; ++k) s = add3(s, mul3(xyz(__ldg(&fwdS[list[k * ls]])), sims[k]));
+    for (uint32_t k = 0; k < n; ++k) s = add3(s, mul3(xyz(ldStep<CHAIN>(&fwdS[list[k * ls]])), sims[k]));
     if (n > 0) s = mul3(normalize3(sub3(div3(s, (float)n), a.fwd)), fl.aclus);
     steer = add3(s, steer);
   }
@@ -1032,6 +1035,7 @@ __device__ __forceinline__ f3 obstacleSteer(const AgentCtx& a, const FlockDev& f
 
 // Feature relaxation toward the similarity-weighted neighbour mean (no
 // reference counterpart; the similarity is the reference's computeSimilarity).
+template <bool CHAIN>
 __device__ __forceinline__ void relaxFeatures(const FlockDev& fl, const uint32_t* list, uint32_t ls, uint32_t n, const float* fi,
                                               float norm1, const float* __restrict__ featS, uint32_t Fs, float* fo) {
   for (uint32_t k = 0; k < fl.F; ++k) fo[k] = fi[k];
@@ -1041,9 +1045,9 @@ __device__ __forceinline__ void relaxFeatures(const FlockDev& fl, const uint32_t
   for (uint32_t k = 0; k < fl.F; ++k) acc[k] = 0.0f;
   for (uint32_t m = 0; m < n; ++m) {
     const float* fj = featS + (size_t)list[m * ls] * Fs;
-    const float s = similarity(fi, norm1, fj, fl.F);
+    const float s = similarity<CHAIN>(fi, norm1, fj, fl.F);
     sumS += s;
-    for (uint32_t k = 0; k < fl.F; ++k) acc[k] += s * __ldg(&fj[k]);
+    for (uint32_t k = 0; k < fl.F; ++k) acc[k] += s * ldStep<CHAIN>(&fj[k]);
   }
   if (sumS > 0.0f) {
     for (uint32_t k = 0; k < fl.F; ++k) {

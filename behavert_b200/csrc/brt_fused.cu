@@ -61,13 +61,13 @@ __host__ __device__ constexpr size_t flockSmemBytes(uint32_t block, uint32_t Mma
 // two sums are independent of the others', so all of it belongs in that one
 // pass: each neighbour's features are read once instead of twice, its norm comes
 // with its position, and no similarity is stored.
-template <int FP, int P2, bool CLUS = false>
+template <bool CHAIN, int FP, int P2, bool CLUS = false>
 __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const float4 p4, const FlockDev& fl,
                                           const uint32_t* list, uint32_t ls, uint32_t n) {
   const f3 p = xyz(p4);
   // Phase 2: steering and feature sums over the list, in list order.
-  const float4 w4 = __ldg(&A.fwdS[i]);
-  const float4 a4 = __ldg(&A.accS[i]);
+  const float4 w4 = ldStep<CHAIN>(&A.fwdS[i]);
+  const float4 a4 = ldStep<CHAIN>(&A.accS[i]);
   const f3 fwd = xyz(w4);
   const bool cosFree = dot3(fwd, fwd) * 1.002f < fl.cosBound2;
   const bool sepOn = fl.sep[0] != 0.0f, aliOn = fl.ali[0] != 0.0f, cohOn = fl.coh[0] != 0.0f;
@@ -81,7 +81,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
     const float4* src = reinterpret_cast<const float4*>(A.featS) + (size_t)i * fs4;
 #pragma unroll
     for (int q = 0; q < FP / 4; ++q) {
-      const float4 v = (uint32_t)q < fs4 ? __ldg(&src[q]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 v = (uint32_t)q < fs4 ? ldStep<CHAIN>(&src[q]) : make_float4(0.f, 0.f, 0.f, 0.f);
       fi[4 * q + 0] = v.x; fi[4 * q + 1] = v.y; fi[4 * q + 2] = v.z; fi[4 * q + 3] = v.w;
     }
 #pragma unroll
@@ -132,7 +132,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
   float4 stats = make_float4(0.f, 0.f, 0.f, 0.f);
   uint32_t id = 0;
   if (CLUS && clusOn) {
-    id = __ldg(&A.idS[i]);
+    id = ldStep<CHAIN>(&A.idS[i]);
     stats = A.statsById[id];
   }
   auto visitFeat = [&](const float* fj, float n2, uint32_t j, const float4 q4) {
@@ -161,7 +161,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
           const f3 seek = sub3(to, myVel), flee = sub3(mk3(-to.x, -to.y, -to.z), myVel);
           sClus = add3(sClus, add3(mul3(seek, sim), mul3(flee, 1.0f - sim)));
         }
-        if (clusAli) sClusAli = add3(sClusAli, mul3(xyz(__ldg(&A.fwdS[j])), sim));
+        if (clusAli) sClusAli = add3(sClusAli, mul3(xyz(ldStep<CHAIN>(&A.fwdS[j])), sim));
       }
     }
   };
@@ -174,7 +174,7 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
       const float4* src = reinterpret_cast<const float4*>(A.featS) + (size_t)j * fs4;
 #pragma unroll
       for (int qq = 0; qq < FP / 4; ++qq) {
-        const float4 v = (uint32_t)qq < fs4 ? __ldg(&src[qq]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v = (uint32_t)qq < fs4 ? ldStep<CHAIN>(&src[qq]) : make_float4(0.f, 0.f, 0.f, 0.f);
         fj[4 * qq + 0] = v.x; fj[4 * qq + 1] = v.y; fj[4 * qq + 2] = v.z; fj[4 * qq + 3] = v.w;
       }
     }
@@ -183,11 +183,11 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
   if (P2 == 0) {
     for (uint32_t k = 0; k < n; ++k) {
       const uint32_t j = list[k * ls];
-      const float4 q = __ldg(&A.posS[j]);
+      const float4 q = ldStep<CHAIN>(&A.posS[j]);
       float fj[FP > 0 ? FP : 1];
       float n2 = q.w;  // the neighbour's feature norm
       loadFeat(j, fj);
-      visit(q, aliOn ? __ldg(&A.fwdS[j]) : zero4, fj, n2);
+      visit(q, aliOn ? ldStep<CHAIN>(&A.fwdS[j]) : zero4, fj, n2);
     }
   } else if (P2 == 2) {
     // Two walks over the list, geometry first, then the feature sums: every
@@ -195,14 +195,14 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
     // keeps only its own accumulators live.
     for (uint32_t k = 0; k < n; ++k) {
       const uint32_t j = list[k * ls];
-      visitGeom(__ldg(&A.posS[j]), aliOn ? __ldg(&A.fwdS[j]) : zero4);
+      visitGeom(ldStep<CHAIN>(&A.posS[j]), aliOn ? ldStep<CHAIN>(&A.fwdS[j]) : zero4);
     }
     if (relaxOn || clusOn) {
       for (uint32_t k = 0; k < n; ++k) {
         const uint32_t j = list[k * ls];
         float fj[FP > 0 ? FP : 1];
         loadFeat(j, fj);
-        const float4 q = __ldg(&A.posS[j]);
+        const float4 q = ldStep<CHAIN>(&A.posS[j]);
         visitFeat(fj, q.w, j, q);
       }
     }
@@ -211,8 +211,8 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
       const bool two = k + 1 < n;
       const uint32_t j0 = list[k * ls];
       const uint32_t j1 = two ? (list[(k + 1) * ls]) : j0;
-      const float4 q0 = __ldg(&A.posS[j0]), q1 = __ldg(&A.posS[j1]);
-      const float4 w0 = aliOn ? __ldg(&A.fwdS[j0]) : zero4, w1 = aliOn ? __ldg(&A.fwdS[j1]) : zero4;
+      const float4 q0 = ldStep<CHAIN>(&A.posS[j0]), q1 = ldStep<CHAIN>(&A.posS[j1]);
+      const float4 w0 = aliOn ? ldStep<CHAIN>(&A.fwdS[j0]) : zero4, w1 = aliOn ? ldStep<CHAIN>(&A.fwdS[j1]) : zero4;
       float f0[FP > 0 ? FP : 1], f1[FP > 0 ? FP : 1];
       float n20 = q0.w, n21 = q1.w;
       loadFeat(j0, f0);
@@ -261,15 +261,19 @@ __device__ __forceinline__ void flockWalk(const FusedArgs& A, uint32_t i, const 
     for (int q = 0; q < FP / 4; ++q)
       if ((uint32_t)q < fs4) dst[q] = make_float4(fi[4 * q], fi[4 * q + 1], fi[4 * q + 2], fi[4 * q + 3]);
   }
+  if constexpr (CHAIN) id = ldStep<CHAIN>(&A.idS[i]);  // before the stores that an ordinary load is not moved across
   const Integrated r = integrate(a, a4, steer, A.dt, fl);
   A.posA[i] = r.pos;
   A.fwdA[i] = r.fwd;
   A.accA[i] = r.acc;
-  A.idA[i] = __ldg(&A.idS[i]);
+  if constexpr (!CHAIN) id = ldStep<CHAIN>(&A.idS[i]);
+  A.idA[i] = id;
 }
 
-template <int FP, int P2, int MINB, int SCAN, bool CLUS = false>
+template <int FP, int P2, int MINB, int SCAN, bool CLUS = false, bool CHAIN = false>
 __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs A) {
+  // (the per-agent scans read with __ldg)
+  static_assert(!CHAIN || SCAN >= 4, "only the cooperative scans have chained instantiations");
   extern __shared__ __align__(16) uint32_t sFlock[];
   chainBegin();
   uint32_t* sList = sFlock + (SCAN >= 4 && SCAN != 9 ? (blockDim.x >> 5) * kSegments * 4u : 0u);
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs 
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
   const FlockDev& fl = A.flocks[f];
-  const float4 p4 = __ldg(&A.posS[i]);
+  const float4 p4 = ldStep<CHAIN>(&A.posS[i]);
   const f3 p = xyz(p4);
   const uint32_t G = fl.G;
   // The plain quotient here (the same cell as gridCoord's product): measured,
@@ -305,19 +309,19 @@ __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs 
     float4* segs = reinterpret_cast<float4*>(sFlock) + (threadIdx.x >> 5) * kSegments;
     if constexpr (SCAN == 7) {
       float4* cbuf = reinterpret_cast<float4*>(sList + cullBufOffsetWords(ls, A.Mmax)) + (threadIdx.x >> 5) * kCullBufPerWarp;
-      n = scanNeighborsCooperative<kCoopCachedRounds, 0, true>(active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd,
+      n = scanNeighborsCooperative<CHAIN, kCoopCachedRounds, 0, true>(active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd,
                                                                A.posS, sList, ls, threadIdx.x & ~31u, segs, cbuf);
     } else if constexpr (SCAN >= 8) {
       float* dList = reinterpret_cast<float*>(sList + ls * A.Mmax);
-      n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents, false, true, SCAN == 9>(
+      n = scanNeighborsCooperative<CHAIN, kCoopCachedRounds, kCoopWindowAgents, false, true, SCAN == 9>(
           active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u, segs, nullptr, dList);
     } else {
-      n = scanNeighborsCooperative<kCoopCachedRounds, SCAN == 5 ? kCoopWindowAgents : 0>(
+      n = scanNeighborsCooperative<CHAIN, kCoopCachedRounds, SCAN == 5 ? kCoopWindowAgents : 0>(
           active, i, p, key, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u, segs);
     }
     if (!active) return;
   } else {
-    const bool cull = A.cullGate && __ldg(A.cullGate) == 0u;
+    const bool cull = A.cullGate && ldStep<CHAIN>(A.cullGate) == 0u;
     n = A.scanVariant == 0 ? scanNeighborsPipelined<4, true>(i, p, fl, A.cellStart, A.cellEnd, A.posS, list, ls, cull)
       : A.scanVariant == 1 ? scanNeighborsPipelined<2, true>(i, p, fl, A.cellStart, A.cellEnd, A.posS, list, ls, cull)
       : A.scanVariant == 2 ? scanNeighborsPipelined<4, false>(i, p, fl, A.cellStart, A.cellEnd, A.posS, list, ls, false)
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(kFlockMaxThreads, MINB) flockKernel(FusedArgs 
     for (uint32_t k = 0; k < n; ++k) out[1 + k] = list[k * ls];
   }
 
-  flockWalk<FP, P2, CLUS>(A, i, p4, fl, list, ls, n);
+  flockWalk<CHAIN, FP, P2, CLUS>(A, i, p4, fl, list, ls, n);
 }
 
 // Exclusive scan of one value per thread across a kTileThreads block.
@@ -516,7 +520,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
         const bool inTile = gx >= (int)x0 && gx < (int)(x0 + R) && gy == (int)ty && gz == (int)tz;
         if (active && inTile) n = scanTileStaged(i, p, gx, gy, gz, x0, W, fl, sStage, sOff, sCnt, sList + tid, ls);
       } else {
-        n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, homeCell(gx, gy, gz, fl), A.flocks,
+        n = scanNeighborsCooperative<false, kCoopCachedRounds, kCoopWindowAgents>(active, i, p, homeCell(gx, gy, gz, fl), A.flocks,
                                                                             f, A.cellStart, A.cellEnd, A.posS, sList, ls,
                                                                             tid & ~31u, sSegs + (tid >> 5) * kSegments);
       }
@@ -527,7 +531,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
           out[0] = n;
           for (uint32_t k = 0; k < n; ++k) out[1 + k] = list[k * ls];
         }
-        flockWalk<FP, P2>(A, i, p4, fl, list, ls, n);
+        flockWalk<false, FP, P2>(A, i, p4, fl, list, ls, n);
       }
       __syncwarp();
     }
@@ -551,27 +555,36 @@ inline uint32_t clusBlocks(uint32_t features4, uint32_t n) {
 // 1619 / 1338.
 constexpr int walk2Blocks(int FP) { return FP > 16 ? 2 : (FP > 8 ? 3 : 4); }
 namespace {
+// Chained instantiations exist for the default launch options alone: other
+// options run in full order at every size.
+template <int SCAN>
+constexpr bool kChainedScan = SCAN == 5 || SCAN == 8 || SCAN == 9;
 template <int FP, int SCAN>
 cudaError_t launchFlockScan(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
                      cudaStream_t st) {
   if constexpr (SCAN == 0) {
     if (phase2 == 1) {
-      if (regs > 64) return launchChained(A.n, flockKernel<FP, 1, 2, 0>, blocks, block, smem, st, A);
-      else return launchChained(A.n, flockKernel<FP, 1, 4, 0>, blocks, block, smem, st, A);
+      if (regs > 64) return launchPlain(flockKernel<FP, 1, 2, 0>, blocks, block, smem, st, A);
+      else return launchPlain(flockKernel<FP, 1, 4, 0>, blocks, block, smem, st, A);
     }
   }
   if constexpr (SCAN >= 4 && FP > 0) {
     if (phase2 == 2) {
-      if (regs <= 48) return launchChained(A.n, flockKernel<FP, 2, 5, SCAN>, blocks, block, smem, st, A);
-      else return launchChained(A.n, flockKernel<FP, 2, walk2Blocks(FP), SCAN>, blocks, block, smem, st, A);
+      if (regs <= 48) return launchPlain(flockKernel<FP, 2, 5, SCAN>, blocks, block, smem, st, A);
+      if constexpr (kChainedScan<SCAN>)
+        return launchChainedOr(A.n, flockKernel<FP, 2, walk2Blocks(FP), SCAN, false, true>,
+                               flockKernel<FP, 2, walk2Blocks(FP), SCAN>, blocks, block, smem, st, A);
+      else return launchPlain(flockKernel<FP, 2, walk2Blocks(FP), SCAN>, blocks, block, smem, st, A);
     }
   }
   if constexpr (SCAN >= 4) {
-    if (regs <= 40) return launchChained(A.n, flockKernel<FP, 0, 6, SCAN>, blocks, block, smem, st, A);
-    if (regs <= 48) return launchChained(A.n, flockKernel<FP, 0, 5, SCAN>, blocks, block, smem, st, A);
+    if (regs <= 40) return launchPlain(flockKernel<FP, 0, 6, SCAN>, blocks, block, smem, st, A);
+    if (regs <= 48) return launchPlain(flockKernel<FP, 0, 5, SCAN>, blocks, block, smem, st, A);
   }
-  if (regs > 64) return launchChained(A.n, flockKernel<FP, 0, 2, SCAN>, blocks, block, smem, st, A);
-  else return launchChained(A.n, flockKernel<FP, 0, 4, SCAN>, blocks, block, smem, st, A);
+  if (regs > 64) return launchPlain(flockKernel<FP, 0, 2, SCAN>, blocks, block, smem, st, A);
+  if constexpr (FP == 0 && kChainedScan<SCAN>)
+    return launchChainedOr(A.n, flockKernel<0, 0, 4, SCAN, false, true>, flockKernel<0, 0, 4, SCAN>, blocks, block, smem, st, A);
+  else return launchPlain(flockKernel<FP, 0, 4, SCAN>, blocks, block, smem, st, A);
 }
 template <int FP>
 cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, size_t smem, int phase2, int regs,
@@ -579,9 +592,10 @@ cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, s
   if constexpr (FP > 0) {
     if constexpr (FP <= 8) {
       if (A.clus && clusBlocks(A.Fs, A.n) == 3u)
-        return launchChained(A.n, flockKernel<FP, 2, 3, 5, true>, blocks, block, smem, st, A);
+        return launchPlain(flockKernel<FP, 2, 3, 5, true>, blocks, block, smem, st, A);
     }
-    if (A.clus) return launchChained(A.n, flockKernel<FP, 2, 2, 5, true>, blocks, block, smem, st, A);
+    if (A.clus)
+      return launchChainedOr(A.n, flockKernel<FP, 2, 2, 5, true, true>, flockKernel<FP, 2, 2, 5, true>, blocks, block, smem, st, A);
   }
   if (A.scanVariant == 4) return launchFlockScan<FP, 4>(A, blocks, block, smem, phase2, regs, st);
   else if (A.scanVariant == 5) return launchFlockScan<FP, 5>(A, blocks, block, smem, phase2, regs, st);
@@ -595,6 +609,12 @@ cudaError_t configureCoopScan(int smem) {
   const void* fns[4] = {(const void*)flockKernel<FP, 0, 4, SCAN>, (const void*)flockKernel<FP, 0, 2, SCAN>,
                         (const void*)flockKernel<FP, 0, 5, SCAN>, (const void*)flockKernel<FP, 0, 6, SCAN>};
   for (const void* fn : fns) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  if constexpr (kChainedScan<SCAN>) {
+    constexpr int walk = FP > 0 ? 2 : 0;
+    const void* fn = (const void*)flockKernel<FP, walk, walk2Blocks(FP), SCAN, false, true>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
@@ -620,6 +640,8 @@ cudaError_t configureFlockFP(int smem, int smemCull, int smemKnn) {
   if constexpr (FP > 0) {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(flockKernel<FP, 2, 2, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(flockKernel<FP, 2, 2, 5, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if constexpr (FP <= 8) {
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(flockKernel<FP, 2, 3, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -169,11 +169,27 @@ __device__ __forceinline__ uint32_t flockOfSlotInWarp(const uint32_t* __restrict
 // slots that are free early, so the ones that work later are unevenly spread and
 // other streams' blocks find no room (65,536 agents 55 -> 65 us; three kNN engines
 // of 262,144 in turn 396 -> 697).  8,192 agents: 28.5 / 27.7, with features 51.6 / 53.0.
+//
+// A chained kernel reads what the step's other kernels write with ordinary loads
+// (ldStep<true>), not with __ldg: a non-coherent load asks for memory that nothing
+// writes while the kernel exists, and a chained kernel's blocks exist while their
+// predecessor writes; the compiler may also move such a load up past the wait, which
+// orders ordinary accesses only.  Kernels that also run unchained come in two
+// instantiations: with ordinary loads everywhere the 1,024-flock batch's step takes
+// 3,780 instead of 3,656 us (place +20%, reorder +11%, flock +3%: loads the compiler
+// may not move across stores and votes).  __ldg stays for the tables that only the
+// host and kernels in full order write (agentBase, obstacles, obsMask, tiles).
 constexpr uint32_t kChainAgents = 5000;
+template <bool CHAIN, class T>
+__device__ __forceinline__ T ldStep(const T* p) {
+  if constexpr (CHAIN) return *p;
+  else return __ldg(p);
+}
 __device__ __forceinline__ void chainBegin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// A kernel that reads nothing of a step by ldStep, chained or not.
 template <class... P, class... Q>
 inline cudaError_t launchChained(uint32_t agents, void (*kernel)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st,
                                  Q&&... args) {
@@ -188,6 +204,17 @@ inline cudaError_t launchChained(uint32_t agents, void (*kernel)(P...), dim3 gri
   cfg.attrs = &attr;
   cfg.numAttrs = agents <= kChainAgents ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// The chained instantiation of a kernel in a small engine, else the plain one.
+template <class... P, class... Q>
+inline cudaError_t launchChainedOr(uint32_t agents, void (*chained)(P...), void (*plain)(P...), dim3 grid, uint32_t block,
+                                   size_t smem, cudaStream_t st, Q&&... args) {
+  return launchChained(agents, agents <= kChainAgents ? chained : plain, grid, block, smem, st, args...);
+}
+// Never chained: a launch in full order.
+template <class... P, class... Q>
+inline cudaError_t launchPlain(void (*kernel)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st, Q&&... args) {
+  return launchChained(kChainAgents + 1, kernel, grid, block, smem, st, args...);
 }
 
 // ---------------------------------------------------------------------------

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) hashKernel(HashArgs A) {
 // order by counting: thread i's agent is member i of its cell, in no order; its
 // sorted position is the cell's first plus the members with smaller ids (the
 // members of a cell of more than kRankLimit are in id order already).
-template <bool RANK>
+template <bool RANK, bool CHAIN>
 __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
   chainBegin();
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,17 +76,17 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
     uint32_t key, ps, i = t;
     uint32_t prev = 0, next = 0;
     if constexpr (RANK) {
-      const uint4 m = __ldg(&A.members[t]);
+      const uint4 m = ldStep<CHAIN>(&A.members[t]);
       ps = m.y;
       key = m.w;
       const uint32_t s = m.z;
       // (a stale entry, left by a step whose waits ran out, must stay in bounds)
       if (ps >= A.n || key >= A.numCells || s > t) { atomicOr(A.errWord, kDevErrOrder); continue; }
-      const uint32_t e = __ldg(&A.cellEnd[key]);
+      const uint32_t e = ldStep<CHAIN>(&A.cellEnd[key]);
       if (e > A.n || e <= t) { atomicOr(A.errWord, kDevErrOrder); continue; }
       if (e - s <= kRankLimit) {
         i = s;
-        for (uint32_t q = s; q < e; ++q) i += __ldg(&A.members[q].x) < m.x ? 1u : 0u;
+        for (uint32_t q = s; q < e; ++q) i += ldStep<CHAIN>(&A.members[q].x) < m.x ? 1u : 0u;
       }
       A.pairsOut[i] = make_uint2(key, ps);
     } else {
@@ -97,10 +97,18 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
       prev = i > 0 ? A.pairs[i - 1].x : kEmpty;
       next = i + 1 < A.n ? A.pairs[i + 1].x : kEmpty;
     }
-    float4 pos = __ldg(&A.posA[ps]);
-    A.fwdS[i] = __ldg(&A.fwdA[ps]);
-    A.accS[i] = __ldg(&A.accA[ps]);
-    A.idS[i] = __ldg(&A.idA[ps]);
+    float4 pos = ldStep<CHAIN>(&A.posA[ps]);
+    if constexpr (CHAIN) {  // an ordinary load is not moved across a store
+      const float4 fwd = ldStep<CHAIN>(&A.fwdA[ps]), acc = ldStep<CHAIN>(&A.accA[ps]);
+      const uint32_t id = ldStep<CHAIN>(&A.idA[ps]);
+      A.fwdS[i] = fwd;
+      A.accS[i] = acc;
+      A.idS[i] = id;
+    } else {
+      A.fwdS[i] = ldStep<CHAIN>(&A.fwdA[ps]);
+      A.accS[i] = ldStep<CHAIN>(&A.accA[ps]);
+      A.idS[i] = ldStep<CHAIN>(&A.idA[ps]);
+    }
     if (A.prevOut) A.prevOut[i] = ps;
     if (A.fs4) {
       // The feature norm sqrtf(sum f^2) (computeSimilarity's norma,
@@ -112,8 +120,16 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
       const float4* src = reinterpret_cast<const float4*>(A.featA) + (size_t)ps * A.fs4;
       float4* dst = reinterpret_cast<float4*>(A.featS) + (size_t)i * A.fs4;
       float nn = 0.0f;
+      float4 next;  // chained: one load ahead of the store, as above
+      if constexpr (CHAIN) next = ldStep<CHAIN>(&src[0]);
       for (uint32_t q = 0; q < A.fs4; ++q) {
-        const float4 v = __ldg(&src[q]);
+        float4 v;
+        if constexpr (CHAIN) {
+          v = next;
+          if (q + 1 < A.fs4) next = ldStep<CHAIN>(&src[q + 1]);
+        } else {
+          v = ldStep<CHAIN>(&src[q]);
+        }
         dst[q] = v;
         nn += v.x * v.x;
         nn += v.y * v.y;
@@ -157,9 +173,10 @@ struct AgentOut {
   Integrated r;
 };
 
+template <bool CHAIN>
 __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, uint32_t Fs, uint32_t i, uint32_t F, float* fi) {
   const float* src = featS + (size_t)i * Fs;
-  for (uint32_t k = 0; k < F; ++k) fi[k] = __ldg(&src[k]);
+  for (uint32_t k = 0; k < F; ++k) fi[k] = ldStep<CHAIN>(&src[k]);
 }
 
 // The list-first kernel (option "two_pass", kNN lists above a warp, kNN and
@@ -169,7 +186,7 @@ __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, ui
 // come from the warp-cooperative windowed scan (every lane of a warp takes
 // part; inactive lanes mirror the last agent read-only and leave after it),
 // kNN lists (maxNeighbors above a warp) from the per-agent scan.
-template <bool KNN>
+template <bool KNN, bool CHAIN>
 __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   extern __shared__ uint32_t sList[];
   __shared__ float4 sSegs[KNN ? 1 : kFusedThreads / 32 * kSegments];
@@ -180,23 +197,23 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   const uint32_t i = active ? i0 : A.n - 1;
   const uint32_t f = A.nflocks == 1 ? 0u : flockOfSlot(A.agentBase, A.nflocks, i);
   const FlockDev& fl = A.flocks[f];
-  const float4 p4 = __ldg(&A.posS[i]);
+  const float4 p4 = ldStep<CHAIN>(&A.posS[i]);
   uint32_t* list = sList + threadIdx.x;
   const uint32_t ls = blockDim.x + 1;
   uint32_t n;
   if constexpr (KNN) {
     float distL[BRT_MAX_NEIGHBORS];
-    n = buildNeighborList<true>(i, xyz(p4), fl, A.cellStart, A.cellEnd, A.posS, list, ls, distL);
+    n = buildNeighborList<CHAIN, true>(i, xyz(p4), fl, A.cellStart, A.cellEnd, A.posS, list, ls, distL);
   } else {
     const f3 p = xyz(p4);
     const HomeCell home = homeCell(gridCoord(p.x, fl), gridCoord(p.y, fl), gridCoord(p.z, fl), fl);
-    n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(active, i, p, home, A.flocks, f, A.cellStart,
+    n = scanNeighborsCooperative<CHAIN, kCoopCachedRounds, kCoopWindowAgents>(active, i, p, home, A.flocks, f, A.cellStart,
                                                                       A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u,
                                                                       sSegs + (threadIdx.x >> 5) * kSegments);
     if (!active) return;
   }
-  const float4 w4 = __ldg(&A.fwdS[i]);
-  const float4 a4 = __ldg(&A.accS[i]);
+  const float4 w4 = ldStep<CHAIN>(&A.fwdS[i]);
+  const float4 a4 = ldStep<CHAIN>(&A.accS[i]);
   if (A.lists) {
     uint32_t* out = A.lists + (size_t)i * A.listStride;
     out[0] = n;
@@ -204,25 +221,25 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   }
   const AgentCtx a = makeCtx(p4, w4, fl);
   f3 steer = mk3(0.f, 0.f, 0.f);
-  steer = flockingSteer(a, fl, list, ls, n, A.posS, A.fwdS, steer, fl.sep[0] != 0.0f, fl.ali[0] != 0.0f, fl.coh[0] != 0.0f);
+  steer = flockingSteer<CHAIN>(a, fl, list, ls, n, A.posS, A.fwdS, steer, fl.sep[0] != 0.0f, fl.ali[0] != 0.0f, fl.coh[0] != 0.0f);
   float fi[BRT_MAX_FEATUREDIM];
   float norm1 = 0.0f;
   const uint32_t F = fl.F;
   if (F) {
-    loadFeatures(A.featS, A.Fs, i, F, fi);
+    loadFeatures<CHAIN>(A.featS, A.Fs, i, F, fi);
     norm1 = selfNorm(fi, F);
   }
   if (F && (fl.clus != 0.0f || fl.aclus != 0.0f)) {
-    const uint32_t id = __ldg(&A.idS[i]);
+    const uint32_t id = ldStep<CHAIN>(&A.idS[i]);
     float4 st = A.statsById[id];
     float sims[BRT_MAX_NEIGHBORS];
-    steer = clusteringSteer(a, fl, list, ls, n, A.posS, A.fwdS, fi, norm1, A.featS, A.Fs, st, sims, steer);
+    steer = clusteringSteer<CHAIN>(a, fl, list, ls, n, A.posS, A.fwdS, fi, norm1, A.featS, A.Fs, st, sims, steer);
     A.statsById[id] = st;
   }
   if (fl.numObstacles && fl.obsW != 0.0f) steer = obstacleSteer(a, fl, A.obstacles, A.obsMask, steer);
   if (F) {
     float fo[BRT_MAX_FEATUREDIM];
-    relaxFeatures(fl, list, ls, n, fi, norm1, A.featS, A.Fs, fo);
+    relaxFeatures<CHAIN>(fl, list, ls, n, fi, norm1, A.featS, A.Fs, fo);
     float* dst = A.featA + (size_t)i * A.Fs;
     for (uint32_t k = 0; k < F; ++k) dst[k] = fo[k];
   }
@@ -230,7 +247,7 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
   A.posA[i] = r.pos;
   A.fwdA[i] = r.fwd;
   A.accA[i] = r.acc;
-  A.idA[i] = __ldg(&A.idS[i]);
+  A.idA[i] = ldStep<CHAIN>(&A.idS[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -253,11 +270,11 @@ __global__ void __launch_bounds__(128) listsKernel(StageArgs A) {
   const f3 p = xyz(__ldg(&A.posS[i]));
   if constexpr (KNN) {
     float distL[BRT_MAX_NEIGHBORS];
-    out[0] = buildNeighborList<true>(i, p, fl, A.cellStart, A.cellEnd, A.posS, out + 1, 1, distL);
+    out[0] = buildNeighborList<false, true>(i, p, fl, A.cellStart, A.cellEnd, A.posS, out + 1, 1, distL);
   } else {
     const HomeCell home = homeCell(gridCoord(p.x, fl), gridCoord(p.y, fl), gridCoord(p.z, fl), fl);
     const uint32_t ls = blockDim.x + 1;
-    const uint32_t n = scanNeighborsCooperative<kCoopCachedRounds, kCoopWindowAgents>(
+    const uint32_t n = scanNeighborsCooperative<false, kCoopCachedRounds, kCoopWindowAgents>(
         active, i, p, home, A.flocks, f, A.cellStart, A.cellEnd, A.posS, sList, ls, threadIdx.x & ~31u,
         sSegs + (threadIdx.x >> 5) * kSegments);
     if (!active) return;
@@ -278,17 +295,17 @@ __global__ void __launch_bounds__(128) steerStageKernel(StageArgs A, int which) 
   const AgentCtx a = makeCtx(__ldg(&A.posS[i]), __ldg(&A.fwdS[i]), fl);
   const float4 s4 = A.steer[i];
   f3 steer = xyz(s4);
-  if (which == 0 && fl.sep[0] != 0.0f) steer = flockingSteer(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, true, false, false);
-  if (which == 1 && fl.ali[0] != 0.0f) steer = flockingSteer(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, false, true, false);
-  if (which == 2 && fl.coh[0] != 0.0f) steer = flockingSteer(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, false, false, true);
+  if (which == 0 && fl.sep[0] != 0.0f) steer = flockingSteer<false>(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, true, false, false);
+  if (which == 1 && fl.ali[0] != 0.0f) steer = flockingSteer<false>(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, false, true, false);
+  if (which == 2 && fl.coh[0] != 0.0f) steer = flockingSteer<false>(a, fl, lst + 1, 1, n, A.posS, A.fwdS, steer, false, false, true);
   if (which == 3 && fl.F && (fl.clus != 0.0f || fl.aclus != 0.0f)) {
     float fi[BRT_MAX_FEATUREDIM];
-    loadFeatures(A.featS, A.Fs, i, fl.F, fi);
+    loadFeatures<false>(A.featS, A.Fs, i, fl.F, fi);
     const float norm1 = selfNorm(fi, fl.F);
     const uint32_t id = __ldg(&A.idS[i]);
     float4 st = A.statsById[id];
     float sims[BRT_MAX_NEIGHBORS];
-    steer = clusteringSteer(a, fl, lst + 1, 1, n, A.posS, A.fwdS, fi, norm1, A.featS, A.Fs, st, sims, steer);
+    steer = clusteringSteer<false>(a, fl, lst + 1, 1, n, A.posS, A.fwdS, fi, norm1, A.featS, A.Fs, st, sims, steer);
     A.statsById[id] = st;
   }
   if (which == 4 && fl.numObstacles && fl.obsW != 0.0f) steer = obstacleSteer(a, fl, A.obstacles, A.obsMask, steer);
@@ -326,9 +343,9 @@ __global__ void __launch_bounds__(128) integrateStageKernel(StageArgs A, float d
   const AgentCtx a = makeCtx(p4, w4, fl);
   if (fl.F) {
     float fi[BRT_MAX_FEATUREDIM], fo[BRT_MAX_FEATUREDIM];
-    loadFeatures(A.featS, A.Fs, i, fl.F, fi);
+    loadFeatures<false>(A.featS, A.Fs, i, fl.F, fi);
     const float norm1 = selfNorm(fi, fl.F);
-    relaxFeatures(fl, lst + 1, 1, n, fi, norm1, A.featS, A.Fs, fo);
+    relaxFeatures<false>(fl, lst + 1, 1, n, fi, norm1, A.featS, A.Fs, fo);
     float* dst = A.featA + (size_t)i * A.Fs;
     for (uint32_t k = 0; k < fl.F; ++k) dst[k] = fo[k];
   }
@@ -402,17 +419,20 @@ cudaError_t launchHash(const HashArgs& A, uint32_t smBlocks, cudaStream_t st) {
 }
 cudaError_t launchReorder(const ReorderArgs& A, cudaStream_t st) {
   if (A.members) {
-    return launchChained(A.n, reorderKernel<true>, std::max(1u, blocksFor(A.n, 256)), 256, 0, st, A);
+    return launchChainedOr(A.n, reorderKernel<true, true>, reorderKernel<true, false>, std::max(1u, blocksFor(A.n, 256)), 256, 0,
+                           st, A);
   }
   const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
-  return launchChained(A.n, reorderKernel<false>, blocks, 256, 0, st, A);
+  return launchChainedOr(A.n, reorderKernel<false, true>, reorderKernel<false, false>, blocks, 256, 0, st, A);
 }
 cudaError_t configureFusedKernels(uint32_t Mmax) {
   const int smem = (int)((size_t)(kFusedThreads + 1) * Mmax * 4);
-  cudaError_t e = cudaFuncSetAttribute(fusedKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(fusedKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
+  const void* fns[4] = {(const void*)fusedKernel<true, false>, (const void*)fusedKernel<true, true>,
+                        (const void*)fusedKernel<false, false>, (const void*)fusedKernel<false, true>};
+  for (const void* fn : fns) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
   return cudaFuncSetAttribute(listsKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(129 * Mmax * 4));
 }
 namespace {
@@ -426,7 +446,7 @@ uint32_t residentWarpAgents(const void* fn, int threads, size_t smem, uint32_t n
 }
 }  // namespace
 uint32_t fusedWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
-  return residentWarpAgents((const void*)fusedKernel<false>, kFusedThreads, (size_t)(kFusedThreads + 1) * Mmax * 4, n, smCount);
+  return residentWarpAgents((const void*)fusedKernel<false, false>, kFusedThreads, (size_t)(kFusedThreads + 1) * Mmax * 4, n, smCount);
 }
 uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
   return residentWarpAgents((const void*)listsKernel<false>, 128, (size_t)129 * Mmax * 4, n, smCount);
@@ -434,8 +454,11 @@ uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount) {
 cudaError_t launchFused(const FusedArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const size_t smem = (size_t)(kFusedThreads + 1) * A.Mmax * 4;
-  if (knn) return launchChained(A.n, fusedKernel<true>, blocksFor(A.n, kFusedThreads), kFusedThreads, smem, st, A);
-  return launchChained(A.n, fusedKernel<false>, blocksFor(A.n, kFusedThreads / 32 * A.warpAgents), kFusedThreads, smem, st, A);
+  if (knn)
+    return launchChainedOr(A.n, fusedKernel<true, true>, fusedKernel<true, false>, blocksFor(A.n, kFusedThreads), kFusedThreads,
+                           smem, st, A);
+  return launchChainedOr(A.n, fusedKernel<false, true>, fusedKernel<false, false>,
+                         blocksFor(A.n, kFusedThreads / 32 * A.warpAgents), kFusedThreads, smem, st, A);
 }
 cudaError_t launchLists(const StageArgs& A, bool knn, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;

@@ -78,6 +78,7 @@ __device__ __forceinline__ uint32_t ctaExclusiveScan(uint32_t v, uint32_t* sWarp
 // Agents are in the previous step's order, so neighbouring lanes mostly share
 // a cell: one atomic a run of equal cells (its first lane adds the run's
 // length), about a quarter of one an agent at 4 agents a cell.
+template <bool CHAIN>
 __global__ void __launch_bounds__(256) countKernel(OrderArgs A, uint32_t cellTiles) {
   chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(256) countKernel(OrderArgs A, uint32_t cellTil
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t key = 0xFFFFFFFFu;
   if (j < A.n) {
-    const float4 p = __ldg(&A.pos[j]);
+    const float4 p = ldStep<CHAIN>(&A.pos[j]);
     const FlockDev& fl = A.flocks[A.nflocks == 1 ? 0u : flockOfSlotInWarp(A.agentBase, A.nflocks, j)];
     const int gx = gridCoord(p.x, fl), gy = gridCoord(p.y, fl), gz = gridCoord(p.z, fl);
     key = fl.cellBase + ((uint32_t)gz * fl.G + (uint32_t)gy) * fl.G + (uint32_t)gx;
@@ -263,15 +264,16 @@ __device__ void sortBigCell(const OrderArgs& A, uint32_t s, uint32_t e, uint32_t
   __syncthreads();
 }
 
+template <bool CHAIN>
 __global__ void __launch_bounds__(kPlaceThreads) placeKernel(OrderArgs A, uint32_t blocks) {
   __shared__ bool sLast;
   chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t big = A.words[kOrderWordBig];
   if (j < A.n) {
-    const uint2 kp = __ldg(&A.cellPlace[j]);
-    const uint32_t id = __ldg(&A.id[j]);
-    const uint32_t s = __ldg(&A.cellStart[kp.x]);
+    const uint2 kp = ldStep<CHAIN>(&A.cellPlace[j]);
+    const uint32_t id = ldStep<CHAIN>(&A.id[j]);
+    const uint32_t s = ldStep<CHAIN>(&A.cellStart[kp.x]);
     const uint32_t p = s + kp.y;
     if (s != kEmpty && p < A.n) A.members[p] = make_uint4(id, j, s, kp.x);
     else atomicOr(A.errWord, kDevErrOrder);
@@ -307,7 +309,7 @@ uint32_t orderCellTiles(uint32_t numCells) {
 cudaError_t launchOrderCount(const OrderArgs& A, cudaStream_t st) {
   if (A.n == 0) return cudaSuccess;
   const uint32_t tiles = orderCellTiles(A.numCells);
-  return launchChained(A.n, countKernel, (std::max(A.n, tiles) + 255) / 256, 256, 0, st, A, tiles);
+  return launchChainedOr(A.n, countKernel<true>, countKernel<false>, (std::max(A.n, tiles) + 255) / 256, 256, 0, st, A, tiles);
 }
 
 cudaError_t launchOrderPlace(const OrderArgs& A, cudaStream_t st) {
@@ -322,7 +324,7 @@ cudaError_t launchOrderPlace(const OrderArgs& A, cudaStream_t st) {
   }
   if (e != cudaSuccess) return e;
   const uint32_t blocks = (A.n + kPlaceThreads - 1) / kPlaceThreads;
-  return launchChained(A.n, placeKernel, blocks, kPlaceThreads, 0, st, A, blocks);
+  return launchChainedOr(A.n, placeKernel<true>, placeKernel<false>, blocks, kPlaceThreads, 0, st, A, blocks);
 }
 
 }  // namespace brt
