@@ -441,15 +441,20 @@ int brt_adjoint_forward(brt_engine* e, float elapsedTime, uint32_t nsteps, uint3
   DeviceGuard guard(e->device);
   if (!e->adj) e->adj = new AdjointState();
   AdjointState* a = e->adj;
-  if ((rc = ensureCapacity(e, 1, 0, nsteps, true))) return rc;  // everything but the tape
+  // Storage that could not be had whole is given back: the previous forward's
+  // tape may be gone and arrays missing, and nothing may run on what is left.
+  auto giveBack = [&](int status) {
+    cudaStreamSynchronize(e->stream);
+    freeAdjoint(a);
+    e->adj = nullptr;
+    return status;
+  };
+  if ((rc = ensureCapacity(e, 1, 0, nsteps, true))) return giveBack(rc);  // everything but the tape
   bool whole = wholeTapeFits(e, nsteps);
-  if (whole && ensureCapacity(e, 1, nsteps, nsteps, true)) {
-    cudaGetLastError();  // the memory went to someone else meanwhile: checkpoints
-    whole = false;
-  }
+  if (whole && ensureCapacity(e, 1, nsteps, nsteps, true)) whole = false;  // the memory went to someone else meanwhile
   const uint32_t k = whole ? nsteps : std::min(checkpoint_every, nsteps);
   const uint32_t nck = (nsteps + k - 1) / k;
-  if (!whole && (rc = ensureCapacity(e, nck, k, nsteps, false))) return rc;
+  if (!whole && (rc = ensureCapacity(e, nck, k, nsteps, false))) return giveBack(rc);
   if (a->T != nsteps || a->k != k || a->dt != elapsedTime || a->whole != whole) dropGraphs(a);
   a->whole = whole;
   a->T = nsteps; a->k = k; a->nck = nck; a->dt = elapsedTime;

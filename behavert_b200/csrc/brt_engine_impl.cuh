@@ -129,8 +129,12 @@ template <class T>
 inline int devAlloc(T** p, size_t count) {
   *p = nullptr;
   if (count == 0) return BRT_OK;
-  BRT_CUDA_TRY(cudaMalloc((void**)p, count * sizeof(T)));
-  return BRT_OK;
+  const cudaError_t err = cudaMalloc((void**)p, count * sizeof(T));
+  if (err == cudaSuccess) return BRT_OK;
+  *p = nullptr;
+  cudaGetLastError();  // reported here, not by the next kernel launch
+  setLastError(std::string("cudaMalloc: ") + cudaGetErrorString(err));
+  return BRT_ERR_CUDA;
 }
 
 // Defined in brt_engine.cu.
