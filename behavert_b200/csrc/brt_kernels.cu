@@ -173,6 +173,14 @@ struct AgentOut {
   Integrated r;
 };
 
+// Columns of an agent's features beyond its flock's own (flocks of one engine may
+// differ in featuresCount, and state I/O carries every column) move with the agent.
+template <bool CHAIN>
+__device__ __forceinline__ void carryColumns(const float* __restrict__ featS, float* featA, uint32_t Fs, uint32_t i, uint32_t F) {
+  const size_t row = (size_t)i * Fs;
+  for (uint32_t k = F; k < Fs; ++k) featA[row + k] = ldStep<CHAIN>(&featS[row + k]);
+}
+
 template <bool CHAIN>
 __device__ __forceinline__ void loadFeatures(const float* __restrict__ featS, uint32_t Fs, uint32_t i, uint32_t F, float* fi) {
   const float* src = featS + (size_t)i * Fs;
@@ -243,6 +251,7 @@ __global__ void __launch_bounds__(kFusedThreads) fusedKernel(FusedArgs A) {
     float* dst = A.featA + (size_t)i * A.Fs;
     for (uint32_t k = 0; k < F; ++k) dst[k] = fo[k];
   }
+  carryColumns<CHAIN>(A.featS, A.featA, A.Fs, i, F);
   const Integrated r = integrate(a, a4, steer, A.dt, fl);
   A.posA[i] = r.pos;
   A.fwdA[i] = r.fwd;
@@ -349,6 +358,7 @@ __global__ void __launch_bounds__(128) integrateStageKernel(StageArgs A, float d
     float* dst = A.featA + (size_t)i * A.Fs;
     for (uint32_t k = 0; k < fl.F; ++k) dst[k] = fo[k];
   }
+  carryColumns<false>(A.featS, A.featA, A.Fs, i, fl.F);
   const Integrated r = integrate(a, a4, xyz(A.steer[i]), dt, fl);
   A.posA[i] = r.pos;
   A.fwdA[i] = r.fwd;
