@@ -191,7 +191,7 @@ void freeAll(brt_engine* e) {
     for (int k = 0; k < 5; ++k)
       if (e->ev[r][k]) cudaEventDestroy(e->ev[r][k]);
   void* ptrs[] = {e->flocks, e->agentBase, e->obstacles, e->obsMask, e->posA, e->fwdA, e->accA, e->posS, e->fwdS, e->accS,
-                  e->featA, e->featS, e->idA, e->idS, e->statsById, e->steer, e->lists, e->pairs[0], e->pairs[1],
+                  e->featA, e->featS, e->featOwn, e->idA, e->idS, e->statsById, e->steer, e->lists, e->pairs[0], e->pairs[1],
                   e->cellStart, e->cellEnd, e->sortMem, e->errWord, e->stage4, e->stageF, e->stepCounter, e->cullWords,
                   e->membership[0], e->membership[1], e->cellPlace, e->members, e->orderCount, e->orderMem};
   for (void* p : ptrs)
@@ -309,6 +309,10 @@ int enqueueReorder(brt_engine* e) {
     R.cullWords = e->cullWords;
     R.flocks = e->flocks; R.agentBase = e->agentBase; R.nflocks = e->nflocks;
   }
+  if (e->featOwn) {
+    R.featOwn = e->featOwn;
+    R.flocks = e->flocks; R.agentBase = e->agentBase; R.nflocks = e->nflocks;
+  }
   if (e->orderByCount) {
     R.members = e->members;
     R.pairsOut = e->pairs[e->finalPairs];
@@ -363,7 +367,12 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
                            : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);
   if (e->school) BRT_CUDA_TRY(launchSchool(F, e->stream));
   else if (twoPass) BRT_CUDA_TRY(launchFused(F, e->anyKnn, e->stream));
-  else BRT_CUDA_TRY(launchFlock(F, e->phase2Variant, e->fusedBlock, e->regBudget, e->stream));
+  else {
+    if (e->featOwn) F.featS = e->featOwn;
+    BRT_CUDA_TRY(launchFlock(F, e->phase2Variant, e->fusedBlock, e->regBudget, e->stream));
+    if (e->featOwn)
+      BRT_CUDA_TRY(launchCarryColumns(e->featS, e->featA, e->Fs, e->flocks, e->agentBase, e->nflocks, e->N, e->stream));
+  }
   if (timed) {
     if ((rc = stageMark(e, 4))) return rc;
     e->pending[e->ringPos] = true;
@@ -579,6 +588,11 @@ int brt_engine_create(const brt_params* flocks, uint32_t num_flocks, int device,
   chk(devAlloc(&e->posA, n)); chk(devAlloc(&e->fwdA, n)); chk(devAlloc(&e->accA, n));
   chk(devAlloc(&e->posS, n)); chk(devAlloc(&e->fwdS, n)); chk(devAlloc(&e->accS, n));
   chk(devAlloc(&e->featA, n * e->Fs)); chk(devAlloc(&e->featS, n * e->Fs));
+  // The flock kernel compares agents over all columns, which is right where all
+  // flocks with features have as many; else it reads rows cut to the flocks' own.
+  bool unequal = false;
+  for (const FlockDev& d : e->flocksHost) unequal = unequal || (d.F != 0 && d.F != e->Fmax);
+  if (unequal) chk(devAlloc(&e->featOwn, n * e->Fs));
   chk(devAlloc(&e->idA, n)); chk(devAlloc(&e->idS, n));
   chk(devAlloc(&e->statsById, n));
   chk(devAlloc(&e->steer, n));

@@ -51,6 +51,7 @@ struct brt_engine {
   // state
   float4 *posA = nullptr, *fwdA = nullptr, *accA = nullptr, *posS = nullptr, *fwdS = nullptr, *accS = nullptr;
   float *featA = nullptr, *featS = nullptr;
+  float* featOwn = nullptr;   // ReorderArgs::featOwn, where flocks with features differ in featuresCount
   uint32_t *idA = nullptr, *idS = nullptr;
   float4* statsById = nullptr;
   float4* steer = nullptr;

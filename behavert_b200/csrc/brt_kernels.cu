@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) hashKernel(HashArgs A) {
 // order by counting: thread i's agent is member i of its cell, in no order; its
 // sorted position is the cell's first plus the members with smaller ids (the
 // members of a cell of more than kRankLimit are in id order already).
-template <bool RANK, bool CHAIN>
+template <bool RANK, bool CHAIN, bool OWN = false>
 __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
   chainBegin();
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -116,10 +116,13 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
       // an agent takes part in: compute it once here, in the same order.
       // It also goes into the sorted position's w (no kernel reads the w
       // of a position; integration always writes 1), so the list walk gets
-      // a neighbour's norm with the neighbour's position.
+      // a neighbour's norm with the neighbour's position.  OWN: flocks differ in
+      // featuresCount, and an agent is compared over its flock's own columns.
       const float4* src = reinterpret_cast<const float4*>(A.featA) + (size_t)ps * A.fs4;
       float4* dst = reinterpret_cast<float4*>(A.featS) + (size_t)i * A.fs4;
       float nn = 0.0f;
+      uint32_t own = 0;
+      if constexpr (OWN) own = A.flocks[flockOfSlot(A.agentBase, A.nflocks, i)].F;
       float4 next;  // chained: one load ahead of the store, as above
       if constexpr (CHAIN) next = ldStep<CHAIN>(&src[0]);
       for (uint32_t q = 0; q < A.fs4; ++q) {
@@ -131,6 +134,13 @@ __global__ void __launch_bounds__(256) reorderKernel(ReorderArgs A) {
           v = ldStep<CHAIN>(&src[q]);
         }
         dst[q] = v;
+        if constexpr (OWN) {
+          if (4 * q + 0 >= own) v.x = 0.0f;
+          if (4 * q + 1 >= own) v.y = 0.0f;
+          if (4 * q + 2 >= own) v.z = 0.0f;
+          if (4 * q + 3 >= own) v.w = 0.0f;
+          reinterpret_cast<float4*>(A.featOwn)[(size_t)i * A.fs4 + q] = v;
+        }
         nn += v.x * v.x;
         nn += v.y * v.y;
         nn += v.z * v.z;
@@ -179,6 +189,12 @@ template <bool CHAIN>
 __device__ __forceinline__ void carryColumns(const float* __restrict__ featS, float* featA, uint32_t Fs, uint32_t i, uint32_t F) {
   const size_t row = (size_t)i * Fs;
   for (uint32_t k = F; k < Fs; ++k) featA[row + k] = ldStep<CHAIN>(&featS[row + k]);
+}
+
+__global__ void __launch_bounds__(256) carryColumnsKernel(const float* featS, float* featA, uint32_t Fs, const FlockDev* flocks,
+                                                          const uint32_t* agentBase, uint32_t nflocks, uint32_t n) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) carryColumns<false>(featS, featA, Fs, i, flocks[flockOfSlot(agentBase, nflocks, i)].F);
 }
 
 template <bool CHAIN>
@@ -427,12 +443,22 @@ cudaError_t launchHash(const HashArgs& A, uint32_t smBlocks, cudaStream_t st) {
   hashKernel<<<blocks, 256, A.passes * A.bins * 4, st>>>(A);
   return cudaGetLastError();
 }
+cudaError_t launchCarryColumns(const float* featS, float* featA, uint32_t Fs, const FlockDev* flocks, const uint32_t* agentBase,
+                               uint32_t nflocks, uint32_t n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  carryColumnsKernel<<<blocksFor(n, 256), 256, 0, st>>>(featS, featA, Fs, flocks, agentBase, nflocks, n);
+  return cudaGetLastError();
+}
 cudaError_t launchReorder(const ReorderArgs& A, cudaStream_t st) {
   if (A.members) {
-    return launchChainedOr(A.n, reorderKernel<true, true>, reorderKernel<true, false>, std::max(1u, blocksFor(A.n, 256)), 256, 0,
-                           st, A);
+    const uint32_t blocks = std::max(1u, blocksFor(A.n, 256));
+    if (A.featOwn)
+      return launchChainedOr(A.n, reorderKernel<true, true, true>, reorderKernel<true, false, true>, blocks, 256, 0, st, A);
+    return launchChainedOr(A.n, reorderKernel<true, true>, reorderKernel<true, false>, blocks, 256, 0, st, A);
   }
   const uint32_t blocks = std::max(1u, blocksFor(std::max(A.n, A.histWords), 256));
+  if (A.featOwn)
+    return launchChainedOr(A.n, reorderKernel<false, true, true>, reorderKernel<false, false, true>, blocks, 256, 0, st, A);
   return launchChainedOr(A.n, reorderKernel<false, true>, reorderKernel<false, false>, blocks, 256, 0, st, A);
 }
 cudaError_t configureFusedKernels(uint32_t Mmax) {

@@ -42,6 +42,9 @@ struct ReorderArgs {
   // ranks it takes, and the sorted pairs it writes; null with the radix sort
   const uint4* members;
   uint2* pairsOut;
+  // engines whose flocks differ in featuresCount: the sorted features with only
+  // each flock's own columns, the others zero (null: all flocks own all columns)
+  float* featOwn;
   // cell-cull gate of scan variants 0 and 1 (null: not computed).  Words
   // [0] and [1] are the launch's accumulator and block ticket, both back at
   // zero when the launch ends; [2] is set to nonzero when a sorted position
@@ -232,6 +235,9 @@ cudaError_t launchAdjointSeed(const SeedArgs& A, cudaStream_t st);
 cudaError_t launchAdjointOut(const OutArgs& A, cudaStream_t st);
 
 cudaError_t launchHash(const HashArgs& A, uint32_t maxBlocks, cudaStream_t st);
+// Canonical features of sorted slot i beyond its flock's own columns, from its sorted row.
+cudaError_t launchCarryColumns(const float* featS, float* featA, uint32_t Fs, const FlockDev* flocks, const uint32_t* agentBase,
+                               uint32_t nflocks, uint32_t n, cudaStream_t st);
 cudaError_t launchReorder(const ReorderArgs& A, cudaStream_t st);
 cudaError_t launchFused(const FusedArgs& A, bool knn, cudaStream_t st);
 cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs, cudaStream_t st);

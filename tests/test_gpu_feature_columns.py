@@ -68,3 +68,39 @@ def test_stages(counts):
         for _ in range(3):
             eng.update_stagewise(w.dt)
         _check(eng, _oracle(w, stats, 3))
+
+
+@pytest.mark.parametrize("counts", [(8, 0, 8), (3, 8), (3, 8, 5, 8), (9, 32, 16, 0), (1, 2, 1)])
+@pytest.mark.parametrize("clustering,relax", [(False, 0.05), (True, 0.05), (True, 0.0)])
+def test_single_pass_kernel(counts, clustering, relax):
+    w, stats = _workload(counts, clustering, relax, seed=3)
+    with Engine(w.params) as eng:
+        _start(eng, w, stats)
+        eng.step(w.dt, 3)
+        _check(eng, _oracle(w, stats, 3))
+
+
+@pytest.mark.parametrize("scan,walk,order", [(0, 0, 1), (0, 1, 1), (4, 0, 0), (5, 2, 0), (6, 0, 1), (6, 2, 1), (7, 2, 1)])
+def test_other_scans_and_walks(scan, walk, order):
+    w, stats = _workload((3, 8, 5, 0), False, 0.05, seed=4)
+    with Engine(w.params) as eng:
+        for key, value in (("scan_variant", scan), ("phase2_variant", walk), ("incremental_sort", order)):
+            eng.set_option(key, value)
+        _start(eng, w, stats)
+        eng.step(w.dt, 3)
+        _check(eng, _oracle(w, stats, 3))
+
+
+def test_values_that_are_no_numbers_in_columns_of_no_flock():
+    w, stats = _workload((3, 8, 5), True, 0.05, seed=5)
+    w.feat[:2500, 3:] = np.float32(np.nan)
+    w.feat[4600:, 5:] = np.float32(np.inf)
+    for n_knn in (0, 1):
+        for p in w.params:
+            p.useKnn = n_knn
+            if n_knn:
+                p.clusteringForceParams[0] = p.alignmentClusteringForceParams[0] = 0.0
+        with Engine(w.params) as eng:
+            _start(eng, w, stats)
+            eng.step(w.dt, 3)
+            _check(eng, _oracle(w, stats, 3))
