@@ -269,20 +269,33 @@ OrderArgs orderArgs(brt_engine* e) {
   A.cellStart = e->cellStart; A.cellEnd = e->cellEnd;
   A.members = e->members;
   A.scratch[0] = e->pairs[0]; A.scratch[1] = e->pairs[1];
-  A.words = e->orderMem; A.bigCells = e->orderMem + kOrderWords;
+  A.words = e->orderMem; A.giantCells = e->orderMem + kOrderWords; A.bigCells = A.giantCells + kGiants;
   A.tileStatus = A.bigCells + bigCellCap(e->N);
+  // (a crowded cell has more than kRankLimit agents, so the buffer holds the words:
+  // n / 2 + 1,024 bytes at most, of 16 n)
+  A.giantStatus = reinterpret_cast<uint32_t*>(e->stage4);
   A.stepCounter = e->stepCounter;
   A.errWord = e->errWord;
   A.wait = e->wait;
   return A;
 }
 
+// Whether a step takes its order by counting.  Not in worlds of few cells: with
+// more than about a hundred agents a cell their ranks cost more than the radix
+// sort, which then has few passes.  us of a warm order by counting / by the radix
+// sort, 1,000,000 agents, 64 a cell: 53 / 69, 128: 61 / 68, 256: 81 / 66, 2,000:
+// 131 / 63, 37,037 (27 cells): 103 / 46; 10,000 agents, 64: 20 / 20, 370: 26 / 18.
+// (A crowd in a world with more cells is placeCrowded's, brt_order.cu.)
+constexpr uint64_t kCountPerCell = 128;
+bool ordersByCount(const brt_engine* e) { return e->orderByCount && e->N <= kCountPerCell * e->C; }
+
 // Order and reorder: by counting the cells, or with the radix sort.
 int enqueueReorder(brt_engine* e) {
   cudaStream_t st = e->stream;
   int rc = stageMark(e, 0);
   if (rc) return rc;
-  if (e->orderByCount) {
+  const bool byCount = ordersByCount(e);
+  if (byCount) {
     const OrderArgs O = orderArgs(e);
     BRT_CUDA_TRY(launchOrderCount(O, st));
     if ((rc = stageMark(e, 1))) return rc;
@@ -313,7 +326,7 @@ int enqueueReorder(brt_engine* e) {
     R.featOwn = e->featOwn;
     R.flocks = e->flocks; R.agentBase = e->agentBase; R.nflocks = e->nflocks;
   }
-  if (e->orderByCount) {
+  if (byCount) {
     R.members = e->members;
     R.pairsOut = e->pairs[e->finalPairs];
   }
@@ -608,7 +621,7 @@ int brt_engine_create(const brt_params* flocks, uint32_t num_flocks, int device,
   if (!rc && cudaMalloc(&e->sortMem, sortBytes) != cudaSuccess) { setLastError("sort scratch allocation failed"); rc = BRT_ERR_CUDA; }
   chk(devAlloc(&e->cellPlace, n)); chk(devAlloc(&e->members, n));
   chk(devAlloc(&e->orderCount, e->Cpad));
-  chk(devAlloc(&e->orderMem, kOrderWords + bigCellCap(e->N) + orderCellTiles(e->C)));
+  chk(devAlloc(&e->orderMem, kOrderWords + kGiants + bigCellCap(e->N) + orderCellTiles(e->C)));
   if (rc) { freeAll(e); delete e; return rc; }
   e->ss = carveSortScratch(e->plan, e->sortMem, false);
   cudaStream_t st = e->stream;
@@ -987,7 +1000,7 @@ int brt_engine_stage_times(brt_engine* e, double* ms4, uint64_t* steps, uint32_t
   if (ms4) for (int k = 0; k < 4; ++k) ms4[k] = e->stageMs[k];
   if (steps) *steps = e->timedSteps;
   // count, cell scan, place, or hash and radix passes; reorder, flock
-  if (launches_per_step) *launches_per_step = 2 + (e->orderByCount ? 3 : 1 + e->plan.passes);
+  if (launches_per_step) *launches_per_step = 2 + (ordersByCount(e) ? 3 : 1 + e->plan.passes);
   e->stageMs[0] = e->stageMs[1] = e->stageMs[2] = e->stageMs[3] = 0;
   e->timedSteps = 0;
   return BRT_OK;

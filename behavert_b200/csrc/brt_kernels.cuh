@@ -106,14 +106,25 @@ struct StageArgs {
   const uint32_t* stepCounter;
 };
 
-// The order by counting (brt_order.cu).  A cell of more than kRankLimit agents
-// is sorted by id before the reorder, which otherwise compares each agent's id
-// with its cell's members' (kRankLimit^2 comparisons of one cell then take about
-// as long as the neighbour scan of its agents).
-constexpr uint32_t kRankLimit = 4096;
+// The order by counting (brt_order.cu).  reorderKernel ranks the members of a
+// cell by comparing their ids; those of a cell of more than kRankLimit placeKernel
+// sorts instead.  us of a warm order of 1,000,000 agents ranked / sorted (and by the
+// radix sort): 500 a cell 115 / 132 (63), 700: 145 / 105 (64), 1,000: 188 / 101 (65),
+// 2,000: 324 / 131 (62), 4,000: 1,724 / 158 (60).
+constexpr uint32_t kRankLimit = 512;
+// Of those, the cells of more than giantLimit, at most kGiants, are sorted together
+// by all blocks; a block each sorts the others.  So no block is left with more than
+// 1 / 256 of the agents: 1,000,000 in one cell 95 us (radix sort 43; with one block
+// for every cell above 4,096 it was 14,300), in 27 cells 103 (46; 14,600); 100,000
+// in one cell 38 (22; 1,380).
+constexpr uint32_t kGiants = 256;
+__host__ __device__ constexpr uint32_t giantLimit(uint32_t n) { return n / kGiants > kRankLimit ? n / kGiants : kRankLimit; }
+constexpr uint32_t kGiantTile = 2048;
 __host__ __device__ constexpr uint32_t bigCellCap(uint32_t n) { return n / kRankLimit + 1; }
-constexpr uint32_t kOrderWordTile = 0, kOrderWordDone = 1, kOrderWordBig = 2;  // scan tiles claimed, place blocks done, crowded cells
-constexpr uint32_t kOrderWords = 4;
+// scan tiles claimed, place blocks done, crowded cells of a block each, giant
+// cells, work items claimed
+constexpr uint32_t kOrderWordTile = 0, kOrderWordDone = 1, kOrderWordBig = 2, kOrderWordGiant = 3, kOrderWordItem = 4;
+constexpr uint32_t kOrderWords = 8;
 struct OrderArgs {
   const float4* pos;             // canonical positions
   const uint32_t* id;            // agent id per canonical slot
@@ -124,7 +135,9 @@ struct OrderArgs {
   uint32_t* cellStart; uint32_t* cellEnd;
   uint4* members;                // [n] by cell: (id, canonical slot, cell's first position, cell)
   uint2* scratch[2];             // [n] each: the pair buffers, for crowded cells
+  uint32_t* giantStatus;         // [tiles of kGiantTile agents x kGiants] look-back state, in a staging buffer
   uint32_t* tileStatus;          // [cell tiles] look-back state of the cell scan
+  uint32_t* giantCells;          // [kGiants]
   uint32_t* bigCells;            // [bigCellCap(n)]
   uint32_t* words;               // [kOrderWords]
   uint32_t* stepCounter;         // random-stream step, advanced once per step

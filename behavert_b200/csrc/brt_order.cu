@@ -14,8 +14,8 @@
 //                 is copied to.
 // A cell holds a few agents, so ranking them by comparing ids is cheaper than
 // sorting: four launches take the place of the histogram, the radix passes and
-// the reorder.  Cells of more than kRankLimit agents, where comparing all pairs
-// would not be, are sorted by id by placeKernel's last block.
+// the reorder.  In a crowded cell (more than kRankLimit agents) comparing all pairs
+// would not be: placeKernel sorts those by id.
 //
 // The kernels are bound by latency (small worlds) or by their scattered 4 to 16
 // byte accesses (large ones).  Measured, us of a warm step for all launches
@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(256) countKernel(OrderArgs A, uint32_t cellTil
     A.words[kOrderWordTile] = 0u;
     A.words[kOrderWordDone] = 0u;
     A.words[kOrderWordBig] = 0u;
+    A.words[kOrderWordGiant] = 0u;
+    A.words[kOrderWordItem] = 0u;
     if (A.stepCounter) *A.stepCounter += 1u;
   }
   const uint32_t lane = threadIdx.x & 31u;
@@ -186,8 +188,10 @@ __global__ void __launch_bounds__(THREADS) cellScanKernel(OrderArgs A) {
     run += tot[k];
     stop[k] = tot[k] ? run : kEmpty;
     if (tot[k] > kRankLimit) {
-      const uint32_t b = atomicAdd(&A.words[kOrderWordBig], 1u);
-      if (b < bigCellCap(A.n)) A.bigCells[b] = c0 + k;
+      const bool giant = tot[k] > giantLimit(A.n);
+      const uint32_t b = atomicAdd(&A.words[giant ? kOrderWordGiant : kOrderWordBig], 1u);
+      if (giant && b < kGiants) A.giantCells[b] = c0 + k;
+      if (!giant && b < bigCellCap(A.n)) A.bigCells[b] = c0 + k;
     }
   }
   if constexpr (ITEMS % 4 == 0) {
@@ -211,65 +215,217 @@ __global__ void __launch_bounds__(THREADS) cellScanKernel(OrderArgs A) {
   }
 }
 
+// What a block needs while it sorts crowded cells.
+struct CrowdShared {
+  uint32_t base[kGiants], start[kGiants], end[kGiants], cell[kGiants];
+  uint16_t count[kPlaceThreads / 32][256];
+  uint32_t warp[kPlaceThreads / 32 + 1];
+  uint32_t item;
+};
+static_assert(kPlaceThreads == 256 && kGiants == 256, "a thread per digit and per giant cell");
+
 // One crowded cell's members, sorted by id: a stable radix sort on 8-bit
 // digits by one CTA of kPlaceThreads threads, 256 members at a time, between
-// members (id, slot) and the pair buffers.
-__device__ void sortBigCell(const OrderArgs& A, uint32_t s, uint32_t e, uint32_t key) {
-  __shared__ uint32_t sBase[256];
-  __shared__ uint32_t sCount[kPlaceThreads / 32][256];
+// members (id, slot), a pair buffer and the places, which nobody reads any more.
+__device__ void sortBigCell(const OrderArgs& A, CrowdShared& S, uint32_t s, uint32_t e, uint32_t key) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint2* const buf[2] = {A.cellPlace, A.scratch[1]};
   for (uint32_t i = s + tid; i < e; i += kPlaceThreads) {
     const uint4 m = __ldcg(&A.members[i]);
-    A.scratch[0][i] = make_uint2(m.x, m.y);
+    buf[0][i] = make_uint2(m.x, m.y);
   }
   uint32_t from = 0;
   for (uint32_t shift = 0; shift < 32u && (A.n - 1u) >> shift; shift += 8u, from ^= 1u) {
-    const uint2* in = A.scratch[from];
-    uint2* out = A.scratch[from ^ 1u];
-    sBase[tid] = 0u;
+    const uint2* in = buf[from];
+    uint2* out = buf[from ^ 1u];
+    S.base[tid] = 0u;
     __syncthreads();
-    for (uint32_t i = s + tid; i < e; i += kPlaceThreads) atomicAdd(&sBase[(__ldcg(&in[i]).x >> shift) & 255u], 1u);
+    for (uint32_t i = s + tid; i < e; i += kPlaceThreads) atomicAdd(&S.base[(__ldcg(&in[i]).x >> shift) & 255u], 1u);
     __syncthreads();
-    __shared__ uint32_t sWarp[kPlaceThreads / 32 + 1];
     uint32_t total;
-    const uint32_t excl = ctaExclusiveScan<kPlaceThreads>(sBase[tid], sWarp, &total);
-    sBase[tid] = excl;
+    const uint32_t excl = ctaExclusiveScan<kPlaceThreads>(S.base[tid], S.warp, &total);
+    S.base[tid] = excl;
     for (uint32_t i0 = s; i0 < e; i0 += kPlaceThreads) {
-      for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) sCount[w][tid] = 0u;
+      for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) S.count[w][tid] = 0;
       __syncthreads();
       const uint32_t i = i0 + tid;
       const uint2 m = i < e ? __ldcg(&in[i]) : make_uint2(0u, 0u);
       const uint32_t d = i < e ? (m.x >> shift) & 255u : 256u;
       const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
       const uint32_t rank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
-      if (d < 256u && rank == 0u) sCount[warp][d] = (uint32_t)__popc(peers);
+      if (d < 256u && rank == 0u) S.count[warp][d] = (uint16_t)__popc(peers);
       __syncthreads();
       if (d < 256u) {
-        uint32_t dst = sBase[d] + rank;
-        for (uint32_t w = 0; w < warp; ++w) dst += sCount[w][d];
+        uint32_t dst = S.base[d] + rank;
+        for (uint32_t w = 0; w < warp; ++w) dst += S.count[w][d];
         if (s + dst < e) out[s + dst] = m;
       }
       __syncthreads();
       uint32_t add = 0;
-      for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) add += sCount[w][tid];
-      sBase[tid] += add;
+      for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) add += S.count[w][tid];
+      S.base[tid] += add;
     }
     __threadfence_block();
     __syncthreads();
   }
   for (uint32_t i = s + tid; i < e; i += kPlaceThreads) {
-    const uint2 m = __ldcg(&A.scratch[from][i]);
+    const uint2 m = __ldcg(&buf[from][i]);
     A.members[i] = make_uint4(m.x, m.y, s, key);
   }
   __syncthreads();
 }
 
+// kGiantTile agents in id order, put behind the earlier tiles' in their giant
+// cells: one pass of a stable partition, the tiles' counts handed on as in the
+// radix sort.  scratch[0] holds (giant cell or none, slot) by agent id.
+__device__ void placeGiantTile(const OrderArgs& A, CrowdShared& S, uint32_t tile, uint32_t giants) {
+  constexpr uint32_t kItems = kGiantTile / kPlaceThreads, kNone = kGiants;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t first = tile * kGiantTile + warp * (32u * kItems) + lane;
+  for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) S.count[w][tid] = 0;
+  __syncthreads();
+  uint32_t at[kItems];  // the cell, and the place among the warp's agents of that cell above it
+#pragma unroll
+  for (uint32_t q = 0; q < kItems; ++q) {
+    const uint32_t id = first + q * 32u;
+    const uint32_t g0 = id < A.n ? __ldcg(&A.scratch[0][id]).x : kNone;
+    const uint32_t g = g0 < giants ? g0 : kNone;
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, g);
+    const uint32_t leader = (uint32_t)__ffs(peers) - 1u;
+    uint32_t before = 0;
+    if (lane == leader && g != kNone) {
+      before = S.count[warp][g];
+      S.count[warp][g] = (uint16_t)(before + (uint32_t)__popc(peers));
+    }
+    before = __shfl_sync(0xFFFFFFFFu, before, leader);
+    at[q] = g | (before + (uint32_t)__popc(peers & ((1u << lane) - 1u))) << 16;
+    __syncwarp();
+  }
+  __syncthreads();
+  if (tid < giants) {
+    uint32_t mine = 0;
+    for (uint32_t w = 0; w < kPlaceThreads / 32; ++w) {
+      const uint32_t c = S.count[w][tid];
+      S.count[w][tid] = (uint16_t)mine;
+      mine += c;
+    }
+    uint32_t* status = A.giantStatus + tid;
+    uint32_t before = 0;
+    if (tile > 0) {
+      stRelaxed(&status[(size_t)tile * kGiants], kLookAgg | mine);
+      // earlier tiles were claimed earlier: their blocks run, and publish
+      int p = (int)tile - 1;
+      uint32_t spins = 0;
+      const bool stalled = tile == A.wait.stallTile;
+      for (bool done = false; !done;) {
+        constexpr int kAhead = 4;
+        uint32_t v[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q)
+          v[q] = p >= q ? (stalled ? 0u : ldRelaxed(&status[(size_t)(p - q) * kGiants])) : kLookInc;
+        int used = 0;
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+          const uint32_t f = v[q] & kLookMask;
+          if (done || used < q || f == 0u) continue;
+          before += v[q] & kLookVal;
+          done = f == kLookInc;
+          ++used;
+        }
+        p -= used;
+        if (!done && used < kAhead && ++spins > A.wait.spinLimit) {
+          atomicOr(A.errWord, kDevErrLookback);
+          break;
+        }
+      }
+    }
+    stRelaxed(&status[(size_t)tile * kGiants], kLookInc | ((before + mine) & kLookVal));
+    S.base[tid] = S.start[tid] + before;
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t q = 0; q < kItems; ++q) {
+    const uint32_t id = first + q * 32u, g = at[q] & 0xFFFFu;
+    if (g == kNone) continue;
+    const uint32_t p = S.base[g] + S.count[warp][g] + (at[q] >> 16);
+    if (p < S.end[g]) A.members[p] = make_uint4(id, __ldcg(&A.scratch[0][id]).y, S.start[g], S.cell[g]);
+  }
+  __syncthreads();
+}
+
+// A step with crowded cells: the blocks claim pieces of work in order.  First
+// the places of 256 slots each, as in the other steps, but the agents of giant
+// cells go to an array by id; then tiles of that array; then a crowded cell each.
+// A piece waits for earlier ones only, and those are with blocks that run.
+__device__ __noinline__ void placeCrowded(const OrderArgs& A, CrowdShared& S, uint32_t placeItems, uint32_t crowded, uint32_t giants) {
+  const uint32_t tid = threadIdx.x;
+  giants = min(giants, kGiants);
+  crowded = min(crowded, bigCellCap(A.n));
+  if (tid < giants) {
+    const uint32_t c = A.giantCells[tid];
+    S.cell[tid] = c;
+    S.start[tid] = A.cellStart[c];
+    S.end[tid] = A.cellEnd[c];
+  }
+  const uint32_t tiles = giants ? (A.n + kGiantTile - 1) / kGiantTile : 0u;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) S.item = atomicAdd(&A.words[kOrderWordItem], 1u);
+    __syncthreads();
+    const uint32_t item = S.item;
+    if (item >= placeItems + tiles + crowded) return;
+    if (item < placeItems) {
+      for (uint32_t w = item * kPlaceThreads + tid; w < tiles * kGiants; w += placeItems * kPlaceThreads) A.giantStatus[w] = 0u;
+      const uint32_t j = item * kPlaceThreads + tid;
+      if (j < A.n) {
+        const uint2 kp = A.cellPlace[j];
+        const uint32_t id = A.id[j], s = A.cellStart[kp.x], p = s + kp.y;
+        uint32_t g = kGiants;
+        if (giants && A.cellEnd[kp.x] - s > giantLimit(A.n))
+          for (uint32_t k = 0; k < giants; ++k)
+            if (S.cell[k] == kp.x) g = k;
+        if (giants && id < A.n) A.scratch[0][id] = make_uint2(g, j);
+        if (s != kEmpty && p < A.n) {
+          if (g == kGiants) A.members[p] = make_uint4(id, j, s, kp.x);
+        } else {
+          atomicOr(A.errWord, kDevErrOrder);
+        }
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) atomicAdd(&A.words[kOrderWordDone], 1u);
+      continue;
+    }
+    if (tid == 0) {
+      uint32_t spins = 0;
+      while (ldRelaxed(&A.words[kOrderWordDone]) < placeItems)
+        if (++spins > A.wait.spinLimit) {
+          atomicOr(A.errWord, kDevErrLookback);
+          break;
+        }
+    }
+    __syncthreads();
+    __threadfence();
+    if (item < placeItems + tiles) {
+      placeGiantTile(A, S, item - placeItems, giants);
+    } else {
+      const uint32_t c = A.bigCells[item - placeItems - tiles];
+      const uint32_t s = A.cellStart[c], e = A.cellEnd[c];
+      if (s < e && e <= A.n) sortBigCell(A, S, s, e, c);
+    }
+  }
+}
+
 template <bool CHAIN>
-__global__ void __launch_bounds__(kPlaceThreads) placeKernel(OrderArgs A, uint32_t blocks) {
-  __shared__ bool sLast;
+__global__ void __launch_bounds__(kPlaceThreads, 8) placeKernel(const __grid_constant__ OrderArgs A, uint32_t blocks) {
+  __shared__ CrowdShared sCrowd;
   chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t big = A.words[kOrderWordBig];
+  const uint32_t crowded = A.words[kOrderWordBig], giants = A.words[kOrderWordGiant];
+  if ((crowded | giants) != 0u) {
+    placeCrowded(A, sCrowd, blocks, crowded, giants);
+    return;
+  }
   if (j < A.n) {
     const uint2 kp = ldStep<CHAIN>(&A.cellPlace[j]);
     const uint32_t id = ldStep<CHAIN>(&A.id[j]);
@@ -277,19 +433,6 @@ __global__ void __launch_bounds__(kPlaceThreads) placeKernel(OrderArgs A, uint32
     const uint32_t p = s + kp.y;
     if (s != kEmpty && p < A.n) A.members[p] = make_uint4(id, j, s, kp.x);
     else atomicOr(A.errWord, kDevErrOrder);
-  }
-  if (big == 0u) return;
-  // crowded cells: the last block sorts them once every member is there
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) sLast = atomicAdd(&A.words[kOrderWordDone], 1u) == blocks - 1u;
-  __syncthreads();
-  if (!sLast) return;
-  __threadfence();
-  for (uint32_t b = 0; b < min(big, bigCellCap(A.n)); ++b) {
-    const uint32_t c = __ldcg(&A.bigCells[b]);
-    const uint32_t s = __ldcg(&A.cellStart[c]), e = __ldcg(&A.cellEnd[c]);
-    if (s < e && e <= A.n) sortBigCell(A, s, e, c);
   }
 }
 
