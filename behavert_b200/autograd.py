@@ -36,8 +36,10 @@ def flock_loss(engine, weights, pos0, vel0, target, dt: float, nsteps: int, chec
 
     weights: [nflocks, 3] float32 CUDA; pos0, vel0, target: [N, 3] float32
     CUDA in agent-id order.  Differentiable in weights, pos0 and vel0; the
-    backward recomputes every checkpoint segment (hash, sort, neighbour
-    lists) and runs the hand-written adjoint kernel.
+    backward runs the hand-written adjoint kernels over the steps' tape, which
+    the forward keeps, or which is computed again from a state kept every
+    `checkpoint_every` steps where the whole tape takes too much memory (the
+    engine option "adjoint_checkpoints" says when, and 1 always recomputes).
     """
     return _ext().flock_loss(int(engine.handle.value), weights, pos0, vel0, target, float(dt), int(nsteps),
                              int(checkpoint_every))

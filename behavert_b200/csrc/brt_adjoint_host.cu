@@ -16,6 +16,8 @@
 // final state of the forward.
 #include "brt_engine_impl.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <string>
 
@@ -24,6 +26,8 @@ namespace brt {
 void setLastError(const std::string& msg);
 
 struct AdjointState {
+  int device = 0;
+  size_t held = 0;            // this engine's part of gTapeBytes
   uint32_t T = 0, k = 0, nck = 0;
   float dt = 0.0f;
   bool taped = false;
@@ -70,15 +74,6 @@ struct AdjointState {
   // graphs: (kind, T, k, dt bits, params version, variant bits)
   std::map<std::tuple<int, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t>, cudaGraphExec_t> graphs;
 };
-
-void freeAdjoint(AdjointState* a) {
-  if (!a) return;
-  for (auto& kv : a->graphs) cudaGraphExecDestroy(kv.second);
-  for (void* p : a->mem) cudaFree(p);
-  for (cudaEvent_t ev : a->events) cudaEventDestroy(ev);
-  if (a->revStream) cudaStreamDestroy(a->revStream);
-  delete a;
-}
 
 namespace {
 
@@ -128,23 +123,58 @@ int checkSupported(brt_engine* e) {
   return BRT_OK;
 }
 
+// Bytes of whole tapes held on each device, all engines together: they share the
+// eighth of its memory that wholeTapeFits allows.
+constexpr int kMaxDevices = 64;
+std::atomic<size_t> gTapeBytes[kMaxDevices];
+
+// Sets the engine's part of gTapeBytes, unless that would exceed `limit`.
+bool holdTape(AdjointState* a, size_t bytes, size_t limit) {
+  if (a->device < 0 || a->device >= kMaxDevices) return bytes == 0;
+  if (bytes > a->held) {
+    const size_t more = bytes - a->held;
+    if (gTapeBytes[a->device].fetch_add(more) + more > limit) {
+      gTapeBytes[a->device].fetch_sub(more);
+      return false;
+    }
+  } else {
+    gTapeBytes[a->device].fetch_sub(a->held - bytes);
+  }
+  a->held = bytes;
+  return true;
+}
+
+// Bytes a step of a tape takes, bytes of a checkpoint, and of everything else.
+size_t tapeStepBytes(const brt_engine* e) { return (size_t)e->N * (4 * 16 + 2 * 4 + 4 * (size_t)e->listStride); }
+size_t checkpointBytes(const brt_engine* e) { return (size_t)e->N * (3 * 16 + 4); }
+size_t adjointBaseBytes(const brt_engine* e) {
+  const size_t perEntry = 2 * 16 + 4, inCap = std::min(64u, 2u * e->Mmax);
+  return (size_t)e->N * (17 * 16 + 3 * 4 + 3 * 8 + 4 * (size_t)e->Fs + perEntry * e->Mmax + 2 * 16 * inCap);
+}
+
 // Whether the forward keeps every step's sorted state and lists instead of
-// checkpoints, so that the backward has nothing to compute again: when they
-// take at most an eighth of the device's memory, and at most half of what is
-// free beside the tape's present size.  Measured with the recompute beside the
-// reverse on a second stream / without it: 65,536 agents x 50 steps (0.4 GB)
-// 8.9 / 6.9 ms forward and backward, 64 flocks of 499 k agents x 40 (2.5 GB)
-// 39.0 / 31.0 ms.
-bool wholeTapeFits(brt_engine* e, uint32_t T) {
+// checkpoints, so that the backward has nothing to compute again: when the
+// adjoint's storage is then at most kTapeGrowth times what the caller's
+// checkpoint distance asks for, the whole tapes of all engines take at most an
+// eighth of the device's memory, and this one at most half of what is free beside
+// the tape's present size.  Measured with the recompute beside the reverse on a
+// second stream / without it: 65,536 agents x 50 steps (0.4 GB) 8.9 / 6.9 ms
+// forward and backward, 64 flocks of 499 k agents x 40 (2.5 GB) 39.0 / 31.0 ms.
+// Horizons of a few dozen steps, every 5 to 10, come to 1.5 to 2.5 times.
+constexpr size_t kTapeGrowth = 3;
+bool wholeTapeFits(brt_engine* e, uint32_t T, uint32_t every) {
+  AdjointState* a = e->adj;
   if (e->adjointCheckpoints) return false;
-  if (T <= e->adj->capK[0]) return true;  // there already
-  const size_t step = (size_t)e->N * (4 * 16 + 2 * 4 + 4 * (size_t)e->listStride);
+  const size_t step = tapeStepBytes(e), base = adjointBaseBytes(e), k = std::min(every, T);
+  const size_t asked = base + (T + k - 1) / k * checkpointBytes(e) + (k < T ? 2 : 1) * k * step;
+  if (T <= a->capK[0]) return true;  // there already
+  if (base + step * T > kTapeGrowth * asked || step * T > e->totalMem / 8) return false;
   size_t freeBytes = 0, total = 0;
   if (cudaMemGetInfo(&freeBytes, &total) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return step * T <= total / 8 && step * T <= (freeBytes + step * e->adj->capK[0]) / 2;
+  return step * T <= (freeBytes + step * a->capK[0]) / 2 && holdTape(a, step * T, e->totalMem / 8);
 }
 
 // (Re)allocates the checkpoint and tape storage for nck checkpoints and k
@@ -220,7 +250,9 @@ int ensureCapacity(brt_engine* e, uint32_t nck, uint32_t k, uint32_t T, bool who
     c.add(&t.prev, n * k);
     c.add(&t.id, n * k);
     c.add(&t.lists, n * k * e->listStride);
+    if (i == 0 && !whole) holdTape(a, 0, 0);
     if ((rc = regrow(&t.mem, c.bytes))) {
+      if (i == 0) holdTape(a, 0, 0);
       dropGraphs(a);
       return rc;
     }
@@ -454,6 +486,33 @@ __global__ void getWeightsKernel(const FlockDev* flocks, float* w, uint32_t nflo
 }
 
 }  // namespace
+
+void freeAdjoint(AdjointState* a) {
+  if (!a) return;
+  holdTape(a, 0, 0);
+  for (auto& kv : a->graphs) cudaGraphExecDestroy(kv.second);
+  for (void* p : a->mem) cudaFree(p);
+  for (cudaEvent_t ev : a->events) cudaEventDestroy(ev);
+  if (a->revStream) cudaStreamDestroy(a->revStream);
+  delete a;
+}
+
+// Gives a tape kept for the whole horizon back (the next forward keeps checkpoints).
+int dropWholeTape(brt_engine* e) {
+  AdjointState* a = e->adj;
+  if (!a || !a->held) return BRT_OK;
+  BRT_CUDA_TRY(cudaStreamSynchronize(e->stream));
+  dropGraphs(a);
+  AdjointState::Tape& t = a->tape[0];
+  a->mem.erase(std::remove(a->mem.begin(), a->mem.end(), (void*)t.mem), a->mem.end());
+  cudaFree(t.mem);
+  t = AdjointState::Tape();
+  a->capK[0] = 0;
+  a->taped = false;
+  holdTape(a, 0, 0);
+  return BRT_OK;
+}
+
 }  // namespace brt
 
 using namespace brt;
@@ -469,7 +528,10 @@ int brt_adjoint_forward(brt_engine* e, float elapsedTime, uint32_t nsteps, uint3
   int rc = checkSupported(e);
   if (rc) return rc;
   DeviceGuard guard(e->device);
-  if (!e->adj) e->adj = new AdjointState();
+  if (!e->adj) {
+    e->adj = new AdjointState();
+    e->adj->device = e->device;
+  }
   AdjointState* a = e->adj;
   // Storage that could not be had whole is given back: the previous forward's
   // tape may be gone and arrays missing, and nothing may run on what is left.
@@ -480,7 +542,7 @@ int brt_adjoint_forward(brt_engine* e, float elapsedTime, uint32_t nsteps, uint3
     return status;
   };
   if ((rc = ensureCapacity(e, 1, 0, nsteps, true))) return giveBack(rc);  // everything but the tape
-  bool whole = wholeTapeFits(e, nsteps);
+  bool whole = wholeTapeFits(e, nsteps, checkpoint_every);
   if (whole && ensureCapacity(e, 1, nsteps, nsteps, true)) whole = false;  // the memory went to someone else meanwhile
   const uint32_t k = whole ? nsteps : std::min(checkpoint_every, nsteps);
   const uint32_t nck = (nsteps + k - 1) / k;

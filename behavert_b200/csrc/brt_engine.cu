@@ -586,7 +586,10 @@ int brt_engine_create(const brt_params* flocks, uint32_t num_flocks, int device,
   e->Fs = (e->Fmax + 3) & ~3u;
   e->listStride = e->Mmax + 1;
   cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) e->smCount = prop.multiProcessorCount;
+  if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) {
+    e->smCount = prop.multiProcessorCount;
+    e->totalMem = prop.totalGlobalMem;
+  }
   uint32_t bits = 1;
   while ((1ull << bits) < C) ++bits;
   e->plan = makeSortPlan(e->N, bits, 8);
@@ -773,6 +776,10 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     e->adjointExport = value != 0;
   } else if (k == "adjoint_checkpoints") {
     e->adjointCheckpoints = value != 0;
+    if (e->adjointCheckpoints) {
+      const int rc = dropWholeTape(e);
+      if (rc) return rc;
+    }
   } else if (k == "lookback_spin_limit") {
     if (value < 0 || value > 0x7FFFFFFFll) { setLastError("lookback_spin_limit must be in [0, 2^31)"); return BRT_ERR_ARG; }
     e->wait.spinLimit = (uint32_t)value;

@@ -10,9 +10,11 @@
 #include <tuple>
 #include <vector>
 
+struct brt_engine;
 namespace brt {
 struct AdjointState;
 void freeAdjoint(AdjointState* a);
+int dropWholeTape(brt_engine* e);
 }  // namespace brt
 
 struct brt_engine {
@@ -80,6 +82,7 @@ struct brt_engine {
   uint32_t paramsVersion = 0;
   std::map<std::tuple<uint32_t, uint32_t, bool, uint32_t>, cudaGraphExec_t> graphs;
   uint32_t smCount = 148;
+  size_t totalMem = 0;  // of the device
   // per-stage timing: a ring of event sets, drained into totals
   static constexpr int kRing = 32;
   bool timing = false, capturing = false;

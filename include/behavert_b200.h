@@ -215,10 +215,14 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p);
                               resident warps and apply to scan_variant 4, 5, 7)
      "adjoint_graphs"   0/1   capture the adjoint forward/backward as graphs (default 1)
      "adjoint_checkpoints" 0/1  1: brt_adjoint_forward always keeps checkpoints
-                              and the backward computes their segments again;
-                              0 (default): it keeps every step's tape where
-                              that takes at most an eighth of the device's
-                              memory and half of what is free
+                              and the backward computes their segments again,
+                              and a tape that is held is freed; 0 (default):
+                              it keeps every step's tape where the adjoint's
+                              storage is then at most three times what
+                              checkpoint_every asks for, the tapes of all
+                              engines take at most an eighth of the device's
+                              memory, and this one half of what is free.  A
+                              tape is held until the engine is destroyed
      "adjoint_export"   0/1   keep the frozen lists and branch flags (brt_adjoint_get_tape)
      "random_step"      uint32 the step counter of the Schooling random stream
                               (every hash pass adds 1 before the move reads it)
