@@ -421,15 +421,21 @@ __global__ void __launch_bounds__(kPlaceThreads, 8) placeKernel(const __grid_con
   __shared__ CrowdShared sCrowd;
   chainBegin();
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t crowded = A.words[kOrderWordBig], giants = A.words[kOrderWordGiant];
-  if ((crowded | giants) != 0u) {
-    placeCrowded(A, sCrowd, blocks, crowded, giants);
+  // (the counts of crowded cells arrive beside the loads that most steps need)
+  static_assert(kOrderWordGiant == kOrderWordBig + 1 && kOrderWordBig % 2 == 0, "read as a pair");
+  const uint2 crowds = *reinterpret_cast<const uint2*>(&A.words[kOrderWordBig]);
+  uint2 kp = make_uint2(0u, 0u);
+  uint32_t id = 0, s = 0;
+  if (j < A.n) {
+    kp = ldStep<CHAIN>(&A.cellPlace[j]);
+    id = ldStep<CHAIN>(&A.id[j]);
+    s = ldStep<CHAIN>(&A.cellStart[kp.x]);
+  }
+  if ((crowds.x | crowds.y) != 0u) {
+    placeCrowded(A, sCrowd, blocks, crowds.x, crowds.y);
     return;
   }
   if (j < A.n) {
-    const uint2 kp = ldStep<CHAIN>(&A.cellPlace[j]);
-    const uint32_t id = ldStep<CHAIN>(&A.id[j]);
-    const uint32_t s = ldStep<CHAIN>(&A.cellStart[kp.x]);
     const uint32_t p = s + kp.y;
     if (s != kEmpty && p < A.n) A.members[p] = make_uint4(id, j, s, kp.x);
     else atomicOr(A.errWord, kDevErrOrder);
