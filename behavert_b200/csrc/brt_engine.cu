@@ -346,6 +346,25 @@ int enqueueReorder(brt_engine* e) {
   return stageMark(e, 3);
 }
 
+// The kernel that takes an engine's steps after the order, and its scan.  The
+// single-pass kernel covers every flock unless one needs kNN lists longer than a
+// warp, or some need kNN and some clustering steering.  kNN flocks take its
+// cooperative kNN scan (scan 8 or 9), clustering ones its scan 5.
+struct StepKernel {
+  enum Kind { kSchool, kListFirst, kFlock } kind;
+  bool clus;
+  int scan;
+};
+StepKernel stepKernel(const brt_engine* e) {
+  StepKernel k{StepKernel::kFlock, false, e->scanVariant};
+  for (const FlockDev& d : e->flocksHost) k.clus = k.clus || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
+  if (e->school) k.kind = StepKernel::kSchool;
+  else if (e->forceTwoPass || (e->anyKnn && (e->Mmax > 32 || k.clus))) k.kind = StepKernel::kListFirst;
+  else if (e->anyKnn) k.scan = flockKnnScan(e->fusedBlock, e->Mmax, e->regBudget);
+  else if (k.clus) k.scan = 5;
+  return k;
+}
+
 int enqueueStep(brt_engine* e, float dt, bool record) {
   const bool timed = e->timing && !e->capturing;
   if (timed) {
@@ -367,19 +386,15 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   F.tiles = e->tiles; F.numTiles = e->numTiles; F.tileCounter = e->tileCounter; F.tileBlocks = e->tileBlocks;
   F.stepCounter = e->stepCounter;
   F.cullGate = (e->scanVariant == 0 || e->scanVariant == 1) ? e->cullWords + 2 : nullptr;
-  // The single-pass kernel covers every flock unless one needs kNN lists longer
-  // than a warp, or some need kNN and some clustering steering.  kNN flocks
-  // take its cooperative kNN scan (scan 8 or 9), clustering ones its scan 5.
-  for (const FlockDev& d : e->flocksHost) F.clus = F.clus || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
-  const bool twoPass = e->forceTwoPass || (e->anyKnn && (e->Mmax > 32 || F.clus));
-  if (!twoPass && F.clus) F.scanVariant = 5;
-  if (e->anyKnn && !twoPass) F.scanVariant = flockKnnScan(e->fusedBlock, e->Mmax, e->regBudget);
+  const StepKernel K = stepKernel(e);
+  F.clus = K.clus;
+  F.scanVariant = K.scan;
   F.steerOut = e->tapeSteer;
-  F.warpAgents = e->school ? e->schoolWarp
-                 : twoPass ? e->fusedWarp
-                           : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);
-  if (e->school) BRT_CUDA_TRY(launchSchool(F, e->stream));
-  else if (twoPass) BRT_CUDA_TRY(launchFused(F, e->anyKnn, e->stream));
+  F.warpAgents = K.kind == StepKernel::kSchool      ? e->schoolWarp
+                 : K.kind == StepKernel::kListFirst ? e->fusedWarp
+                                                    : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);
+  if (K.kind == StepKernel::kSchool) BRT_CUDA_TRY(launchSchool(F, e->stream));
+  else if (K.kind == StepKernel::kListFirst) BRT_CUDA_TRY(launchFused(F, e->anyKnn, e->stream));
   else {
     if (e->featOwn) F.featS = e->featOwn;
     BRT_CUDA_TRY(launchFlock(F, e->phase2Variant, e->fusedBlock, e->regBudget, e->stream));
@@ -750,7 +765,7 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     e->scanVariant = (int)value;
   } else if (k == "incremental_sort") {
     e->orderByCount = value != 0;
-    } else if (k == "block_size") {
+  } else if (k == "block_size") {
     if (value < 32 || value > (int64_t)kFlockMaxThreads || value % 32) {
       setLastError("block_size must be a multiple of 32 in [32, 256]");
       return BRT_ERR_ARG;
@@ -803,7 +818,7 @@ int brt_engine_set_option(brt_engine* e, const char* key, int64_t value) {
     e->ss = carveSortScratch(plan, mem, false);
     e->reordered = false;
     e->listsValid = false;
-    } else {
+  } else {
     setLastError("unknown option " + k);
     return BRT_ERR_ARG;
   }
@@ -1006,8 +1021,11 @@ int brt_engine_stage_times(brt_engine* e, double* ms4, uint64_t* steps, uint32_t
   }
   if (ms4) for (int k = 0; k < 4; ++k) ms4[k] = e->stageMs[k];
   if (steps) *steps = e->timedSteps;
-  // count, cell scan, place, or hash and radix passes; reorder, flock
-  if (launches_per_step) *launches_per_step = 2 + (ordersByCount(e) ? 3 : 1 + e->plan.passes);
+  // count, cell scan, place, or hash and radix passes; reorder, flock (and, where
+  // flocks differ in featuresCount, its other columns)
+  if (launches_per_step)
+    *launches_per_step = 2 + (ordersByCount(e) ? 3 : 1 + e->plan.passes) +
+                         (e->featOwn && stepKernel(e).kind == StepKernel::kFlock ? 1 : 0);
   e->stageMs[0] = e->stageMs[1] = e->stageMs[2] = e->stageMs[3] = 0;
   e->timedSteps = 0;
   return BRT_OK;
@@ -1076,9 +1094,11 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
     *msPerStep = best;
     return BRT_OK;
   };
-  // The flock kernel's options only matter when that kernel runs.
-  bool twoPass = e->anyKnn || e->forceTwoPass || e->school;
-  for (const FlockDev& d : e->flocksHost) twoPass = twoPass || (d.F > 0 && (d.clus != 0.0f || d.aclus != 0.0f));
+  // Which options matter depends on the kernel that takes the steps: none to the
+  // Schooling and list-first kernels; the block size to the clustering steering;
+  // the block size, the walk and the registers to kNN; all of them to the rest.
+  const StepKernel K = stepKernel(e);
+  const bool flock = K.kind == StepKernel::kFlock;
   std::string log;
   char buf[256];
   auto trial = [&](const char* what, int64_t v, double* ms) -> int {
@@ -1087,9 +1107,8 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
     log += buf;
     return r;
   };
-  // Coordinate descent: radix digit width, then block size x scan loop
-  // shape, then the list-walk variant (the last two only when the
-  // single-pass kernel runs).
+  // Coordinate descent: radix digit width, then the flock kernel's options, then
+  // the order by counting against the radix sort.
   uint32_t bestBits = e->plan.digitBits;
   double bestMs = 1e30, ms = 0.0;
   // digit widths only matter with the radix sort
@@ -1105,13 +1124,30 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
   uint32_t bestBlock = e->fusedBlock;
   int bestScan = e->scanVariant, bestP2 = e->phase2Variant;
   int bestRegs = e->regBudget;
-  if (!twoPass) {
+  bool anyFeatures = false;
+  for (const FlockDev& d : e->flocksHost) anyFeatures = anyFeatures || (d.F > 0 && d.relax != 0.0f);
+  const uint32_t blocks[3] = {64, 128, 256};
+  if (flock && (K.clus || e->anyKnn)) {
+    bestMs = 1e30;
+    for (uint32_t bs : blocks)
+      for (int p2 = 0; p2 <= 2 && !rc; p2 += 2) {
+        if (p2 == 2 && (K.clus || !anyFeatures)) continue;
+        chk(brt_engine_set_option(e, "block_size", bs));
+        if (!K.clus) chk(brt_engine_set_option(e, "phase2_variant", p2));
+        if (!rc) chk(trial(K.clus ? "block_size" : (p2 == 2 ? "block_size/walk2" : "block_size/walk0"), bs, &ms));
+        if (!rc && ms < bestMs) { bestMs = ms; bestBlock = bs; bestP2 = K.clus ? bestP2 : p2; }
+      }
+    if (!rc) {
+      chk(brt_engine_set_option(e, "block_size", bestBlock));
+      chk(brt_engine_set_option(e, "phase2_variant", bestP2));
+    }
+  }
+  if (flock && !K.clus && !e->anyKnn) {
     bestMs = 1e30;
     // block size x scan loop x list walk, jointly: the best block depends on
     // the walk.  Walk 1 (two neighbours at a time) only exists for the
     // per-agent scans, walk 2 (geometry, then feature sums) for the
     // cooperative scan of flocks with features.
-    const uint32_t blocks[3] = {64, 128, 256};
     // per agent with / without cell culling, warp-cooperative, cooperative
     // with windows, cooperative with bounding-box culling
     const int scans[5] = {0, 2, 4, 5, 7};
@@ -1120,8 +1156,6 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
                                {"block_size/scan4/walk0", "block_size/scan4/walk2"},
                                {"block_size/scan5/walk0", "block_size/scan5/walk2"},
                                {"block_size/scan7/walk0", "block_size/scan7/walk2"}};
-    bool anyFeatures = false;
-    for (const FlockDev& d : e->flocksHost) anyFeatures = anyFeatures || (d.F > 0 && d.relax != 0.0f);
     for (uint32_t bs : blocks)
       for (int s = 0; s < 5 && !rc; ++s)
         for (int w = 0; w < 2 && !rc; ++w) {
@@ -1147,9 +1181,11 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
       chk(brt_engine_set_option(e, "scan_variant", bestScan));
       chk(brt_engine_set_option(e, "phase2_variant", bestP2));
     }
-    // 48 and 40 only change the cooperative scan's build; the tile kernel has one
+  }
+  if (flock && !K.clus) {
+    // 48 and 40 only change the cooperative scans' build; the tile kernel has one
     const int budgets[4] = {64, 128, 48, 40};
-    const int nBudgets = bestScan == 6 ? 0 : (bestScan >= 4 ? 4 : 2);
+    const int scan = stepKernel(e).scan, nBudgets = scan == 6 ? 0 : (scan >= 4 ? 4 : 2);
     bestMs = 1e30;
     for (int r = 0; r < nBudgets && !rc; ++r) {
       chk(brt_engine_set_option(e, "registers", budgets[r]));
@@ -1158,12 +1194,13 @@ int brt_engine_autotune(brt_engine* e, float elapsedTime, uint32_t steps, char* 
     }
     if (!rc) chk(brt_engine_set_option(e, "registers", bestRegs));
   }
-  // the order by counting against the radix sort
+  // the order by counting against the radix sort (one trial where the world has too
+  // few cells for the first)
   {
-    const int start = e->orderByCount ? 1 : 0;
+    const int start = e->orderByCount ? 1 : 0, orders = e->N <= kCountPerCell * e->C ? 2 : 1;
     int bestResort = start;
     bestMs = 1e30;
-    for (int k = 0; k < 2 && !rc; ++k) {
+    for (int k = 0; k < orders && !rc; ++k) {
       const int v = k == 0 ? start : 1 - start;
       chk(brt_engine_set_option(e, "incremental_sort", v));
       if (!rc) chk(trial("incremental_sort", (uint32_t)v, &ms));
