@@ -665,11 +665,11 @@ cudaError_t launchAdjointStep(const AdjointStepArgs& A, cudaStream_t st) {
   if (A.entryStride == 0 || A.entryStride > 32) return cudaErrorInvalidValue;
   if (A.inCap > 8 * kGatherPerLane || !A.steerS) return cudaErrorInvalidValue;
   const auto blocksOf = [&](uint32_t lanes) { return (uint32_t)(((size_t)A.n * lanes + kAdjointThreads - 1) / kAdjointThreads); };
-  // the most lanes whose blocks are resident at once (148 SMs of kAdjointMinBlocks)
-  constexpr uint32_t kWave = 148u * kAdjointMinBlocks;
+  // the most lanes whose blocks are resident at once
+  const uint32_t wave = A.smCount * kAdjointMinBlocks;
   cudaError_t err;
-  if (blocksOf(4) <= kWave) err = launchChained(A.n, adjointStepKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
-  else if (blocksOf(2) <= kWave) err = launchPlain(adjointStepKernel<2>, blocksOf(2), kAdjointThreads, 0, st, A);
+  if (blocksOf(4) <= wave) err = launchChained(A.n, adjointStepKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);
+  else if (blocksOf(2) <= wave) err = launchPlain(adjointStepKernel<2>, blocksOf(2), kAdjointThreads, 0, st, A);
   else err = launchPlain(adjointStepKernel<1>, blocksOf(1), kAdjointThreads, 0, st, A);
   if (err != cudaSuccess) return err;
   if (A.inCap <= 4 * kGatherPerLane) return launchChained(A.n, adjointGatherKernel<4>, blocksOf(4), kAdjointThreads, 0, st, A);

@@ -397,6 +397,7 @@ int enqueueBackward(brt_engine* e, uint32_t variant) {
     for (int s = (int)steps - 1; s >= 0; --s) {
       AdjointStepArgs R;
       std::memset(&R, 0, sizeof(R));
+      R.smCount = e->smCount;
       R.posS = tp.pos + s * n; R.fwdS = tp.fwd + s * n; R.accS = tp.acc + s * n;
       R.steerS = tp.steer + s * n;
       R.lists = tp.lists + s * n * e->listStride; R.listStride = e->listStride;

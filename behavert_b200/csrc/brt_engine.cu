@@ -390,9 +390,10 @@ int enqueueStep(brt_engine* e, float dt, bool record) {
   F.clus = K.clus;
   F.scanVariant = K.scan;
   F.steerOut = e->tapeSteer;
+  F.smCount = e->smCount;
   F.warpAgents = K.kind == StepKernel::kSchool      ? e->schoolWarp
                  : K.kind == StepKernel::kListFirst ? e->fusedWarp
-                                                    : flockWarpAgents(F, e->fusedBlock, e->regBudget, e->smCount);
+                                                    : flockWarpAgents(F, e->fusedBlock, e->phase2Variant, e->regBudget);
   if (K.kind == StepKernel::kSchool) BRT_CUDA_TRY(launchSchool(F, e->stream));
   else if (K.kind == StepKernel::kListFirst) BRT_CUDA_TRY(launchFused(F, e->anyKnn, e->stream));
   else {

@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(kTileThreads, 4) tileFlockKernel(FusedArgs A) 
 // with 2 / 3 / 4: 8 features 4,096 agents 41 / 44 / 47, 65,536: 77 / 81 / 96,
 // 400,000: 366 / 302 / 316; 32 features 4,096: 55 / 78 / 86, 400,000: 580 / 734 / 745.
 // The list-first kernel: 8 features 97, 138, 521; 32 features 206, 2445.
-inline uint32_t clusBlocks(uint32_t features4, uint32_t n) {
-  return features4 > 8u || n <= 148u * 16u * 32u ? 2u : 3u;
+inline uint32_t clusBlocks(uint32_t features4, uint32_t n, uint32_t smCount) {
+  return features4 > 8u || n <= smCount * 16u * 32u ? 2u : 3u;
 }
 // Resident 256-thread blocks an SM of walk 2 at the default register budget: with
 // more features, fewer blocks and fewer spills.  us a step with 4 / 3 / 2 blocks:
@@ -591,7 +591,7 @@ cudaError_t launchFlockFP(const FusedArgs& A, uint32_t blocks, uint32_t block, s
                           cudaStream_t st) {
   if constexpr (FP > 0) {
     if constexpr (FP <= 8) {
-      if (A.clus && clusBlocks(A.Fs, A.n) == 3u)
+      if (A.clus && clusBlocks(A.Fs, A.n, A.smCount) == 3u)
         return launchPlain(flockKernel<FP, 2, 3, 5, true>, blocks, block, smem, st, A);
     }
     if (A.clus)
@@ -699,22 +699,32 @@ uint32_t flockSmemWarps(uint32_t block, uint32_t Mmax, int scan) {
   return (uint32_t)(228u * 1024u / (flockSmemBytes(block, Mmax, scan) + 1024)) * (block / 32u);
 }
 }  // namespace
+// Resident warps an SM at a register budget (flockKernel's launch bounds).
+static uint32_t budgetWarps(int regs) { return regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u)); }
 // The kNN scan with its run segments in shared memory (8), or in registers (9)
 // where the memory would cost a resident block: 262,144 agents, maxNeighbors 16,
 // 30% in blobs 396 / 409 us a step (three engines), maxNeighbors 30, uniform 288
-// (13 blocks an SM) / 260 (14).
+// (13 blocks an SM) / 260 (14).  By the budget's warps also where features leave
+// fewer: by walk2Blocks' (scan 8 then), 50,000 crowded agents with 32 features and
+// maxNeighbors 30 took 12.7 ms a step for 11.8.
 int flockKnnScan(uint32_t block, uint32_t Mmax, int regs) {
-  const uint32_t byRegs = regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+  const uint32_t byRegs = budgetWarps(regs);
   return std::min(byRegs, flockSmemWarps(block, Mmax, 8)) < std::min(byRegs, flockSmemWarps(block, Mmax, 9)) ? 9 : 8;
 }
-// Resident warps: what the register budget allows (flockKernel's launch
-// bounds), or the lists' shared memory.
-uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount) {
-  const uint32_t byRegs = A.clus ? 8u * clusBlocks(A.Fs, A.n)
-                          : regs > 64 ? 16u : (regs > 48 ? 32u : (regs > 40 ? 40u : 48u));
+// Resident warps: what the registers of the instantiation that launchFlock takes,
+// or the lists' shared memory, allow.  us a step of three engines in turn with the
+// budget's warps / with walk2Blocks' : 12 features, 8,192 agents 26.0 / 18.8, 30,000
+// 28.3 / 21.1; 32 features 8,192 30.8 / 22.6, 20,000 29.6 / 23.2 (alone the same).
+// kNN keeps the budget's: its warps' serial replacements make the tail, and fewer
+// agents a warp cut it (12 features, 8,192 crowded agents alone 389 / 627).
+uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int phase2, int regs) {
+  uint32_t byRegs = budgetWarps(regs);
+  if (A.clus) byRegs = 8u * clusBlocks(A.Fs, A.n, A.smCount);
+  else if (A.scanVariant < 8 && A.Fs > 0 && phase2 == 2 && regs > 48) byRegs = 8u * (uint32_t)walk2Blocks((int)A.Fs);
+  else if (A.scanVariant < 8 && A.Fs > 0 && phase2 == 2) byRegs = 40u;
   const uint32_t resident = std::min(byRegs, flockSmemWarps(block, A.Mmax, A.scanVariant));
   // Taped steps (the adjoint's forward) run alone: its caller waits for them.
-  return warpAgentsFor(A.n, smCount * resident / (A.steerOut ? 1u : 2u));
+  return warpAgentsFor(A.n, A.smCount * resident / (A.steerOut ? 1u : 2u));
 }
 
 cudaError_t launchFlock(const FusedArgs& A, int phase2, uint32_t block, int regs, cudaStream_t st) {

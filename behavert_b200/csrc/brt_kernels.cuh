@@ -68,6 +68,7 @@ struct FusedArgs {
   uint32_t listStride;
   uint32_t nflocks, n, Mmax, Fs;
   uint32_t warpAgents;         // agents a warp of a cooperative scan takes (agentOfLane)
+  uint32_t smCount;            // SMs of the device, for the host's rules
   float dt;
   int scanVariant;             // 0: pipelined x4 + cell culling, 1: x2 + culling, 2: x4, 3: flat loop,
                                // 4: warp-cooperative, 5: warp-cooperative with windows,
@@ -167,7 +168,7 @@ inline uint32_t warpAgentsFor(uint32_t n, uint32_t residentWarps) {
   return 32;
 }
 int flockKnnScan(uint32_t block, uint32_t Mmax, int regs);
-uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int regs, uint32_t smCount);
+uint32_t flockWarpAgents(const FusedArgs& A, uint32_t block, int phase2, int regs);
 uint32_t fusedWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
 uint32_t listsWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
 uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
@@ -176,6 +177,7 @@ uint32_t schoolWarpAgents(uint32_t n, uint32_t Mmax, uint32_t smCount);
 // Reverse of one taped step (brt_adjoint.cu).
 constexpr uint32_t kAdjointThreads = 128;
 struct AdjointStepArgs {
+  uint32_t smCount;                                              // of the device, for the host's rule
   const float4* posS; const float4* fwdS; const float4* accS;   // the step's sorted input state
   const float4* steerS;                                          // and the steering force of its forward
   const uint32_t* lists; uint32_t listStride;                    // its neighbour lists (sorted slots)

@@ -334,6 +334,8 @@ cudaError_t launchSortHistogram(const SortPlan& p, const uint2* in, const SortSc
   uint32_t m[4] = {0, 0, 0, 0};
   for (uint32_t k = 0; k < p.passes; ++k) m[k] = passMask(p, k);
   const bool wide = ((uintptr_t)in & 15u) == 0;
+  // (at most four blocks for each of a B200's SMs; there is no engine to ask, and
+  // any grid counts the same)
   uint32_t blocks = std::min<uint32_t>((p.n + (wide ? 511u : 255u)) / (wide ? 512u : 256u), 148u * 4u);
   switch (p.digitBits) {
 #define BRT_HIST_CASE(B) case B: histogramKernel<B><<<blocks, 256, 0, st>>>(in, p.n, p.passes, p.digitBits, m[0], m[1], m[2], m[3], s.hist, errWord, wide); break;
