@@ -394,7 +394,10 @@ __global__ void __launch_bounds__(128) integrateStageKernel(StageArgs A, float d
 // three launches of 2.5 us -> one of 3.
 // Gather: slot i takes agent id[i]'s values (positions keep w = 1, like the
 // reference's position feature; the features' padding is zero).  Scatter: agent
-// id[i] gets slot i's.
+// id[i] gets slot i's.  A row of single floats is gathered in pieces of a float4 of
+// the padded canonical row.  us of a set call, an agent a thread / a float a thread /
+// so: 1,000,000 agents with 3 features 49.9 / 53.7 / 48.4, 9: 99.3 / 88.9 / 59.2;
+// 4,000,000 with 3: 173 / 202 / 164, 9: 349 / 373 / 235.
 template <bool GATHER, bool WIDE>
 __global__ void __launch_bounds__(256) stateIoKernel(StateIoArgs A) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;  // at most 2^26 agents of 32 features
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(256) stateIoKernel(StateIoArgs A) {
       if (A.src[k]) A.dst[k][to] = v[k];
   }
   // pieces of an agent's features: on the canonical side Fs floats, on the other F
-  const uint32_t per = WIDE ? A.F / 4 : (GATHER ? A.Fs : A.F);
+  const uint32_t per = WIDE || GATHER ? A.Fs / 4 : A.F;
   if (t >= A.n * per) return;
   const uint32_t i = t / per, k = t - i * per;
   const uint32_t id = __ldg(&A.id[i]);
@@ -421,7 +424,10 @@ __global__ void __launch_bounds__(256) stateIoKernel(StateIoArgs A) {
     const size_t slot = (size_t)i * (A.Fs / 4) + k, agent = (size_t)id * per + k;
     dst[GATHER ? slot : agent] = __ldg(&src[GATHER ? agent : slot]);
   } else if (GATHER) {
-    A.featDst[(size_t)i * A.Fs + k] = k < A.F ? __ldg(&A.featSrc[(size_t)id * A.F + k]) : 0.0f;
+    const float* src = A.featSrc + (size_t)id * A.F + 4 * k;
+    const uint32_t left = A.F - 4 * k;
+    reinterpret_cast<float4*>(A.featDst)[(size_t)i * per + k] =
+        make_float4(__ldg(src), left > 1 ? __ldg(src + 1) : 0.0f, left > 2 ? __ldg(src + 2) : 0.0f, left > 3 ? __ldg(src + 3) : 0.0f);
   } else {
     A.featDst[(size_t)id * A.F + k] = __ldg(&A.featSrc[(size_t)i * A.Fs + k]);
   }
@@ -550,7 +556,7 @@ cudaError_t launchStateIoArrays(const StateIoArgs& A, bool gather, cudaStream_t 
   const bool wide = A.featSrc && A.F % 4 == 0 && (((uintptr_t)A.featSrc | (uintptr_t)A.featDst) & 15u) == 0;
   StateIoArgs B = A;
   if (!B.featSrc) B.F = B.Fs = 0;
-  const size_t pieces = (size_t)B.n * (wide ? B.F / 4 : (gather ? B.Fs : B.F));
+  const size_t pieces = (size_t)B.n * (wide || gather ? B.Fs / 4 : B.F);
   const uint32_t blocks = (uint32_t)((std::max<size_t>(B.n, pieces) + 255) / 256);
   if (gather && wide) stateIoKernel<true, true><<<blocks, 256, 0, st>>>(B);
   else if (gather) stateIoKernel<true, false><<<blocks, 256, 0, st>>>(B);
@@ -559,8 +565,11 @@ cudaError_t launchStateIoArrays(const StateIoArgs& A, bool gather, cudaStream_t 
   return cudaGetLastError();
 }
 // Above this many agents each array takes a launch of its own: three streams
-// of scattered 16-byte accesses at once then cost more than the launches save
-// (get, 10.2 M agents: 415 us together, 294 apart; 100,003: 4.2 and 9.3).
+// of scattered 16-byte accesses at once then cost more than the launches save.
+// us of a get call together / apart, no features and 8: 262,144 agents 7.9 / 15.7
+// and 10.2 / 20.3, 600,000: 12.6 / 18.7 and 18.1 / 31.2, 1,000,000: 20.4 / 30.6 and
+// 61.9 / 57.4; 10.2 M: 415 / 294.  (Below about 400,000 the launches' own host time
+// decides.)  The line is on the safe side of where the two cross.
 constexpr uint32_t kStateIoTogether = 1u << 18;
 }  // namespace
 cudaError_t launchStateIo(const StateIoArgs& A, bool gather, cudaStream_t st) {
