@@ -334,8 +334,8 @@ __device__ __forceinline__ float fromOrderedBits(uint32_t u) {
 // segments by counting the segment starts among its 32 positions (one warp-wide
 // OR and a population count) instead of searching the 27 prefixes with five
 // dependent shuffles and five more for the found segment's data.  With the
-// flock's parameters kept from run to run that took a third of the setup's
-// instructions out.
+// flock's parameters kept from run to run: 128 flocks of 1.34 M agents 505 -> 461 us,
+// 385.8 -> 364.6 M warp instructions; 1,048,576 agents with 8 features 643 -> 637 us.
 constexpr uint32_t kSegments = 27;
 // An agent's home cell: the global cell key, and the three coordinates in ten
 // bits each (an engine has at most 2^30 cells).

@@ -168,7 +168,11 @@ __device__ __forceinline__ uint32_t flockOfSlotInWarp(const uint32_t* __restrict
 // all earlier ones ended.  Not in larger engines: blocks that wait take the SM
 // slots that are free early, so the ones that work later are unevenly spread and
 // other streams' blocks find no room (65,536 agents 55 -> 65 us; three kNN engines
-// of 262,144 in turn 396 -> 697).  8,192 agents: 28.5 / 27.7, with features 51.6 / 53.0.
+// of 262,144 in turn 396 -> 697).  us a step plain / chained, alone and three engines
+// in turn: 5,000 agents 38.6 / 36.4 and 14.7 / 14.3, with 8 features 46.5 / 44.2 and
+// 18.2 / 17.8; 7,000: 38.8 / 37.1 and 15.5 / 15.2, 47.3 / 45.1 and 19.3 / 19.3; 16,000:
+// 39.7 / 40.5 and 16.3 / 17.8, 47.6 / 49.0 and 20.6 / 21.9.  The line is a little
+// below where engines side by side gain nothing more.
 //
 // A chained kernel reads what the step's other kernels write with ordinary loads
 // (ldStep<true>), not with __ldg: a non-coherent load asks for memory that nothing

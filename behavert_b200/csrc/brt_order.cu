@@ -23,7 +23,8 @@
 // place, with the hash and radix launches there but gated off): 4,096 agents 13.0
 // against 29; 100,003: 17.7 against 38; 1,048,576 with 8 features: 65 against 87;
 // 1,024 flocks, 10.2 M agents: 385 against 550.  After a changed state, where the
-// radix sort ran: 13 against 30 (4,096), 65 against 108 (1,048,576).
+// radix sort ran: 13 against 30 (4,096), 65 against 108 (1,048,576).  Crowded worlds:
+// kRankLimit; worlds of few cells take the radix sort (ordersByCount).
 #include "brt_kernels.cuh"
 
 #include <algorithm>

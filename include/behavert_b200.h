@@ -179,9 +179,11 @@ int brt_engine_set_params(brt_engine* e, uint32_t flock, const brt_params* p);
      "sort_digit_bits"  4..9  radix digit width of the onesweep passes (default 8;
                               at most 4 passes, so narrow digits on wide keys widen)
      "incremental_sort" 0/1   take the sorted order by counting the agents of
-                              every cell and ranking them by id (default 1),
-                              or with the onesweep radix sort.  The order is
-                              the same either way.
+                              every cell and ranking them by id (default 1;
+                              worlds of more than 128 agents a cell on average
+                              take the radix sort all the same), or with the
+                              onesweep radix sort.  The order is the same
+                              either way.
      "two_pass"         0/1   build each neighbour list before steering even
                               when the single-pass kernel applies (default 0)
      "block_size"       32..256, multiple of 32: threads per block of the
@@ -393,7 +395,7 @@ int brt_engine_check_device_error(brt_engine* e, uint32_t* word);
    brt_reorder_sim_data / brt_compute_neighborhoods, and the state arrays and
    the registered arrays share the sorted order once a step completes.  In an
    engine with features, sorted_pos4's w holds each agent's feature norm
-   (the state's pos4 keeps w = 1).  Kernels may change any value of the
+   over its flock's own columns (the state's pos4 keeps w = 1).  Kernels may change any value of the
    state arrays but must not move agents between slots or rewrite agent_id. */
 #define BRT_MAX_USER_ARRAYS 8
 typedef struct brt_arrays {
