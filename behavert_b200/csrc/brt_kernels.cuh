@@ -120,6 +120,9 @@ constexpr uint32_t kRankLimit = 512;
 // in one cell 38 (22; 1,380).
 constexpr uint32_t kGiants = 256;
 __host__ __device__ constexpr uint32_t giantLimit(uint32_t n) { return n / kGiants > kRankLimit ? n / kGiants : kRankLimit; }
+// Agents a tile of that takes.  us of a warm order with 1,024 / 2,048 / 4,096:
+// 1,000,000 agents in one cell 99 / 103 / 109, in 250 cells (half of them giants)
+// 264 / 166 / 221; 100,000 in 27 cells 40 / 43 / 57.
 constexpr uint32_t kGiantTile = 2048;
 __host__ __device__ constexpr uint32_t bigCellCap(uint32_t n) { return n / kRankLimit + 1; }
 // scan tiles claimed, place blocks done, crowded cells of a block each, giant
